@@ -277,6 +277,10 @@ int omt_bn_apply_pool2(const OmtAct* x, const OmtAct* y, const OmtAct* z, uint8_
 int omt_bn_eval(const OmtAct* x, const OmtAct* y, int32_t n, int32_t c, int32_t h, int32_t w, const float* rm,
                 const float* rv, const float* gamma, const float* beta, float eps, uint32_t flags,
                 omt_stream_t stream);
+/* Eval folding (fold_bn, csrc/fused.cpp:34-40; csrc/plans.cpp:148-160): fw[co][k] = w * scale and
+ * fb[co] = (bias - rm) * scale + beta with scale = gamma * rsqrt(rv + eps); bias may be NULL (0). k = ci * ks * ks. */
+int omt_bn_fold(const float* w, const float* bias, const float* gamma, const float* beta, const float* rm, const float* rv,
+                float eps, int32_t co, int32_t k, float* fw, float* fb, omt_stream_t stream);
 /* Backward (training). dgamma=sum g*xhat, dbeta=sum g, dx=gamma*invstd/m*(m*g-dbeta-xhat*dgamma)
  * (bnb_reduce.wgsl:25-37, bnb_apply.wgsl:19-21). With OMT_BN_RELU, g is first masked by y>0
  * (bn_bwd_part.wgsl:25-38, bn_bwd_apply.wgsl:19-23); y is then required. dx->p may be NULL (mask[0] false).

@@ -161,6 +161,9 @@ bool prefer_cl(const Tensor& x, int64_t co);
 // The same (no ReLU) with the batch-norm partial statistics of y taken in the GEMM epilogue when the call allows it: `groups`
 // is the number of 32-row groups in `partials` (0 and an undefined tensor otherwise; see omt_conv_bnstats_groups).
 Tensor conv_forward_stats(const Tensor& x, const Tensor& w, const Tensor* bias, const OmtConvGeo& g, Tensor& partials, int& groups);
+// eval folding of a BatchNorm into the convolution in front of it (fused.cpp): folded weight and bias
+std::pair<Tensor, Tensor> fold_bn_dev(const Tensor& cw, const std::optional<Tensor>& cb, const Tensor& w, const Tensor& b, const Tensor& rm,
+                                      const Tensor& rv, double eps);
 extern int g_fold;  // eval-plan BN folding (set_fold): 0 off, anything else folds BatchNorm into the conv that feeds it
 
 }  // namespace omt

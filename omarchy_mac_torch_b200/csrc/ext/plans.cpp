@@ -137,10 +137,9 @@ static Tensor plan_forward(Plan& p, const Tensor& x_) {
       bool fold = !p.train && g_fold > 0 && li + 1 < p.layers.size() && p.layers[li + 1].kind == "bn";
       if (fold) {
         const Layer& B = p.layers[li + 1];
-        Tensor scale = p.params[B.param] * at::rsqrt(p.rvs[B.bn] + (double)kEps);
-        Tensor fw = (wt * scale.view({-1, 1, 1, 1})).contiguous();
-        Tensor fb = ((bias ? (*bias - p.rms[B.bn]) : -p.rms[B.bn]) * scale + p.params[B.param + 1]).contiguous();
-        cur = run_conv(cur, fw, &fb, L, true);
+        auto f = fold_bn_dev(wt, bias ? std::optional<Tensor>(*bias) : std::nullopt, p.params[B.param], p.params[B.param + 1], p.rms[B.bn], p.rvs[B.bn],
+                             (double)kEps);
+        cur = run_conv(cur, f.first, &f.second, L, true);
         li++;  // the bn layer is done
       } else if (p.train && L.is_conv() && li + 1 < p.layers.size() && p.layers[li + 1].kind == "bn") {
         // the conv epilogue reduces the BatchNorm's batch statistics while it stores its output

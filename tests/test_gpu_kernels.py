@@ -843,3 +843,19 @@ def test_input_gradient_of_a_first_layer_by_taps(capi, shape, cl):
     assert after.get("conv_dgrad_col2im", 0) == before.get("conv_dgrad_col2im", 0) + 1, after
     exact = capi.conv_dgrad(dev(gy, cl), dev(w), (hw, hw + 2), s, p, flags=capi.FORCE_SIMT)
     assert rel_err(host(got), host(exact)) <= 2e-5
+
+
+@pytest.mark.parametrize("co,ci,ks,bias", [(1, 1, 1, True), (5, 6, 3, False), (64, 3, 7, False), (257, 33, 1, True), (96, 40, 3, True)])
+def test_bn_fold_equals_the_elementwise_ops(capi, co, ci, ks, bias):
+    """omt_bn_fold rounds every product and sum as ATen's elementwise kernels do: the same bits (block edges: 1, 255.. values)."""
+    gen = torch.Generator().manual_seed(co)
+    w = torch.randn(co, ci, ks, ks, generator=gen).cuda()
+    cb = torch.randn(co, generator=gen).cuda() if bias else None
+    gamma, beta, rm = (torch.randn(co, generator=gen).cuda() for _ in range(3))
+    rv = (torch.rand(co, generator=gen) + 1e-3).cuda()
+    fw, fb = torch.empty_like(w), torch.empty_like(gamma)
+    p = capi.ptr
+    capi.call("omt_bn_fold", p(w), p(cb), p(gamma), p(beta), p(rm), p(rv), 1e-5, co, ci * ks * ks, p(fw), p(fb), capi.stream_handle())
+    scale = gamma * torch.rsqrt(rv + 1e-5)
+    assert torch.equal(fw, w * scale.view(-1, 1, 1, 1))
+    assert torch.equal(fb, ((cb - rm) if bias else -rm) * scale + beta)
