@@ -32,6 +32,7 @@ __global__ void __launch_bounds__(256) bn_part_nchw(const float* __restrict__ x,
                                                     const float* __restrict__ y, const uint32_t* __restrict__ bits,
                                                     const float* __restrict__ mean, const float* __restrict__ invstd, int n, int c, int hw, int S,
                                                     float* __restrict__ part) {
+  pdl_wait();
   __shared__ float red[32];
   const int ch = blockIdx.x, sl = blockIdx.y;
   float a0, a1;
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(256) bn_part_nhwc(const float* __restrict__ x,
                                                     const float* __restrict__ y, const uint32_t* __restrict__ bits,
                                                     const float* __restrict__ mean, const float* __restrict__ invstd, int64_t P, int c, int S, int CX,
                                                     float* __restrict__ part) {
+  pdl_wait();
   __shared__ float4 sh1[256], sh2[256];
   const int cx = threadIdx.x % CX, py = threadIdx.x / CX, PY = blockDim.x / CX;
   const int c4 = (blockIdx.x * CX + cx) * 4, sl = blockIdx.y;
@@ -165,6 +167,7 @@ __global__ void __launch_bounds__(256) bn_part_nhwc(const float* __restrict__ x,
 __global__ void __launch_bounds__(256) bn_stats_fin(const float* __restrict__ x, int64_t shift_stride, const float* __restrict__ part, int c, int S,
                                                     float count, float corr, float momentum, float eps, float* mean, float* var, float* invstd,
                                                     const float* rm_in, const float* rv_in, float* rm_out, float* rv_out) {
+  pdl_wait();
   const int ch = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (ch >= c) return;
   float s1 = 0.f, s2 = 0.f;
@@ -188,6 +191,7 @@ __global__ void __launch_bounds__(256) bn_stats_fin(const float* __restrict__ x,
 }
 // finalise backward sums: dgb[0][c] = dgamma (s2), dgb[1][c] = dbeta (s1)   (bn_bwd_fin.wgsl)
 __global__ void __launch_bounds__(256) bn_bwd_fin(const float* __restrict__ part, int c, int S, float scale, float* dgb, float* raw) {
+  pdl_wait();
   const int ch = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (ch >= c) return;
   float s1 = 0.f, s2 = 0.f;
@@ -232,6 +236,7 @@ __device__ __forceinline__ float bn_ew_one(const BnEw& a, float xv, float gv, fl
 
 template <int KIND, bool RELU, bool NHWC>
 __global__ void __launch_bounds__(256) bn_ew_vec4(BnEw a) {
+  pdl_wait();
   int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i >= a.total) return;  // (exited lanes of the last warp: the mask words below then carry unspecified bits past the end, which nobody reads)
   float4 xv = __ldg(reinterpret_cast<const float4*>(a.x + i)), gv = make_float4(0.f, 0.f, 0.f, 0.f), o;
@@ -287,6 +292,7 @@ __global__ void __launch_bounds__(256) bn_ew_vec4(BnEw a) {
 // per 16, and four independent activation loads are in flight per thread. Same arithmetic as bn_ew_vec4.
 template <int KIND, bool RELU>
 __global__ void __launch_bounds__(256) bn_ew_nhwc_px4(BnEw a) {
+  pdl_wait();
   const int c4 = a.c >> 2;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;  // t = pixel group * c4 + channel quad
   const int64_t pg = t < 0x7fffffffll ? (int64_t)((uint32_t)t / (uint32_t)c4) : t / c4;
@@ -345,6 +351,7 @@ __global__ void __launch_bounds__(256) bn_ew_nhwc_px4(BnEw a) {
 
 template <int KIND, bool RELU>
 __global__ void __launch_bounds__(256) bn_ew_scalar(BnEw a, bool nhwc) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.total) return;
   int ch = nhwc ? (int)(i % a.c) : (int)((i / a.hw) % a.c);
@@ -374,21 +381,21 @@ static int launch_ew(const BnEw& a, bool relu, bool nhwc, cudaStream_t s, const 
                    reinterpret_cast<uintptr_t>(a.beta) | reinterpret_cast<uintptr_t>(a.dgb)) & 15) == 0;
   if (vec && nhwc && a.c % 32 == 0 && (a.total / a.c) % 4 == 0) {
     const unsigned blocks = (unsigned)cdiv(a.total / 16, 256);
-    if (relu) bn_ew_nhwc_px4<KIND, true><<<blocks, 256, 0, s>>>(a);
-    else bn_ew_nhwc_px4<KIND, false><<<blocks, 256, 0, s>>>(a);
+    if (relu) launch(bn_ew_nhwc_px4<KIND, true>, blocks, 256, 0, s, a);
+    else launch(bn_ew_nhwc_px4<KIND, false>, blocks, 256, 0, s, a);
   } else if (vec) {
     unsigned blocks = (unsigned)cdiv(a.total / 4, 256);
     if (nhwc) {
-      if (relu) bn_ew_vec4<KIND, true, true><<<blocks, 256, 0, s>>>(a);
-      else bn_ew_vec4<KIND, false, true><<<blocks, 256, 0, s>>>(a);
+      if (relu) launch(bn_ew_vec4<KIND, true, true>, blocks, 256, 0, s, a);
+      else launch(bn_ew_vec4<KIND, false, true>, blocks, 256, 0, s, a);
     } else {
-      if (relu) bn_ew_vec4<KIND, true, false><<<blocks, 256, 0, s>>>(a);
-      else bn_ew_vec4<KIND, false, false><<<blocks, 256, 0, s>>>(a);
+      if (relu) launch(bn_ew_vec4<KIND, true, false>, blocks, 256, 0, s, a);
+      else launch(bn_ew_vec4<KIND, false, false>, blocks, 256, 0, s, a);
     }
   } else {
     unsigned blocks = (unsigned)cdiv(a.total, 256);
-    if (relu) bn_ew_scalar<KIND, true><<<blocks, 256, 0, s>>>(a, nhwc);
-    else bn_ew_scalar<KIND, false><<<blocks, 256, 0, s>>>(a, nhwc);
+    if (relu) launch(bn_ew_scalar<KIND, true>, blocks, 256, 0, s, a, nhwc);
+    else launch(bn_ew_scalar<KIND, false>, blocks, 256, 0, s, a, nhwc);
   }
   return check_launch(name);
 }
@@ -412,6 +419,7 @@ __device__ __forceinline__ void pool4(const float v[4], float& best, int& bi) {
 }
 // channels-last, c % 4 == 0: one thread per output pixel and 4 channels
 __global__ void __launch_bounds__(256) bn_pool2_nhwc4(BnPool a) {
+  pdl_wait();
   const int c4 = a.c >> 2;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)a.n * a.oh * a.ow * c4) return;
@@ -449,6 +457,7 @@ __global__ void __launch_bounds__(256) bn_pool2_nhwc4(BnPool a) {
 // any layout: one thread per output element, in the memory order of z
 template <bool NHWC>
 __global__ void __launch_bounds__(256) bn_pool2_scalar(BnPool a) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)a.n * a.c * a.oh * a.ow) return;
   int img, ch, oy, ox;
@@ -491,16 +500,16 @@ static int launch_part(int lay, const float* x, const float* g, const float* y, 
     int S = (int)std::max<int64_t>(1, std::min<int64_t>(cdiv(P, PY * 4), cdiv(4 * sm_count(), gx)));
     *S_out = S;
     dim3 grid(gx, S);
-    if (relu) bn_part_nhwc<MODE, true><<<grid, 256, 0, s>>>(x, g, y, bits, mean, invstd, P, c, S, CX, part);
-    else bn_part_nhwc<MODE, false><<<grid, 256, 0, s>>>(x, g, y, bits, mean, invstd, P, c, S, CX, part);
+    if (relu) launch(bn_part_nhwc<MODE, true>, grid, 256, 0, s, x, g, y, bits, mean, invstd, P, c, S, CX, part);
+    else launch(bn_part_nhwc<MODE, false>, grid, 256, 0, s, x, g, y, bits, mean, invstd, P, c, S, CX, part);
     return check_launch(MODE == 0 ? "bn_stats_part_nhwc" : "bn_bwd_part_nhwc");
   }
   // NCHW (also used for channels-last with c % 4 != 0 through the caller's layout check)
   int S = (int)std::max<int64_t>(1, std::min<int64_t>(n, cdiv(4 * sm_count(), c)));
   *S_out = S;
   dim3 grid(c, S);
-  if (relu) bn_part_nchw<MODE, true><<<grid, 256, 0, s>>>(x, g, y, bits, mean, invstd, n, c, hw, S, part);
-  else bn_part_nchw<MODE, false><<<grid, 256, 0, s>>>(x, g, y, bits, mean, invstd, n, c, hw, S, part);
+  if (relu) launch(bn_part_nchw<MODE, true>, grid, 256, 0, s, x, g, y, bits, mean, invstd, n, c, hw, S, part);
+  else launch(bn_part_nchw<MODE, false>, grid, 256, 0, s, x, g, y, bits, mean, invstd, n, c, hw, S, part);
   return check_launch(MODE == 0 ? "bn_stats_part_nchw" : "bn_bwd_part_nchw");
 }
 
@@ -535,6 +544,7 @@ __device__ __forceinline__ void merge_lanes(Moments& m, float (*sh)[MERGE_LANES]
     for (int k = 1; k < MERGE_LANES; k++) merge(m, sh[0][k][cx], sh[1][k][cx], sh[2][k][cx]);
 }
 __global__ void __launch_bounds__(32 * MERGE_LANES) bn_partials_kernel(BnFromPartials a) {
+  pdl_wait();
   __shared__ float sh[3][MERGE_LANES][32];
   __shared__ bool last;
   const int cx = threadIdx.x & 31, gl = threadIdx.x >> 5, ch = blockIdx.x * 32 + cx, sl = blockIdx.y, c = a.c;
@@ -595,6 +605,7 @@ static size_t part_floats(int c) { return (size_t)c * (size_t)std::max(8, 4 * sm
 __global__ void __launch_bounds__(256) bn_fold_kernel(const float* __restrict__ w, const float* __restrict__ bias, const float* __restrict__ gamma,
                                                       const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ var,
                                                       float eps, uint32_t total, uint32_t k, float* __restrict__ fw, float* __restrict__ fb) {
+  pdl_wait();
   const uint32_t i = blockIdx.x * 256u + threadIdx.x;
   if (i >= total) return;
   const uint32_t co = i / k;
@@ -630,7 +641,7 @@ int omt_bn_stats(const OmtAct* x, int32_t n, int32_t c, int32_t h, int32_t w, fl
   float count = (float)((int64_t)n * h * w);
   float corr = count / std::max(count - 1.f, 1.f);
   bool fn = flags & OMT_BN_FUNCTIONAL;
-  bn_stats_fin<<<(unsigned)cdiv((int64_t)c * 32, 256), 256, 0, s>>>(x->p, lay == 0 ? (int64_t)h * w : 1, part, c, S, count, corr, momentum, eps,
+  launch(bn_stats_fin, (unsigned)cdiv((int64_t)c * 32, 256), 256, 0, s, x->p, lay == 0 ? (int64_t)h * w : 1, part, c, S, count, corr, momentum, eps,
                                                       mean, var, invstd, rm, rv, rm ? (fn ? new_rm : rm) : nullptr,
                                                       rm ? (fn ? new_rv : rv) : nullptr);
   return check_launch("bn_stats_fin");
@@ -653,7 +664,7 @@ int omt_bn_stats_from_partials(const float* partials, int32_t groups, int32_t c,
   const float* cnt = partials + (size_t)2 * groups * c;
   BnFromPartials a{partials, cnt, reinterpret_cast<unsigned*>(const_cast<float*>(cnt + groups)), (float*)sc.p, groups, c, S, momentum, eps,
                    mean, var, invstd, rm, rv, rm ? (fn ? new_rm : rm) : nullptr, rm ? (fn ? new_rv : rv) : nullptr};
-  bn_partials_kernel<<<dim3(gx, S), 32 * MERGE_LANES, 0, s>>>(a);
+  launch(bn_partials_kernel, dim3(gx, S), 32 * MERGE_LANES, 0, s, a);
   return check_launch("bn_stats_from_partials");
 }
 
@@ -691,9 +702,9 @@ int omt_bn_apply_pool2(const OmtAct* x, const OmtAct* y, const OmtAct* z, uint8_
                    ((reinterpret_cast<uintptr_t>(x->p) | reinterpret_cast<uintptr_t>(a.y.p) | reinterpret_cast<uintptr_t>(z->p) |
                      reinterpret_cast<uintptr_t>(mean) | reinterpret_cast<uintptr_t>(invstd) | reinterpret_cast<uintptr_t>(gamma) |
                      reinterpret_cast<uintptr_t>(beta)) & 15) == 0 && (reinterpret_cast<uintptr_t>(idx) & 3) == 0;
-  if (vec) bn_pool2_nhwc4<<<(unsigned)cdiv(outs / 4, 256), 256, 0, st(stream)>>>(a);
-  else if (lay == 1) bn_pool2_scalar<true><<<(unsigned)cdiv(outs, 256), 256, 0, st(stream)>>>(a);
-  else bn_pool2_scalar<false><<<(unsigned)cdiv(outs, 256), 256, 0, st(stream)>>>(a);
+  if (vec) launch(bn_pool2_nhwc4, (unsigned)cdiv(outs / 4, 256), 256, 0, st(stream), a);
+  else if (lay == 1) launch(bn_pool2_scalar<true>, (unsigned)cdiv(outs, 256), 256, 0, st(stream), a);
+  else launch(bn_pool2_scalar<false>, (unsigned)cdiv(outs, 256), 256, 0, st(stream), a);
   return check_launch("bn_apply_pool2");
 }
 
@@ -712,7 +723,7 @@ int omt_bn_fold(const float* w, const float* bias, const float* gamma, const flo
                 int32_t co, int32_t k, float* fw, float* fb, omt_stream_t stream) {
   OMT_REQUIRE(w && gamma && beta && rm && rv && fw && fb && co > 0 && k > 0 && (int64_t)co * k < (1ll << 31), "omt_bn_fold: bad arguments");
   const uint32_t total = (uint32_t)co * (uint32_t)k;
-  bn_fold_kernel<<<(unsigned)cdiv(total, 256), 256, 0, st(stream)>>>(w, bias, gamma, beta, rm, rv, eps, total, (uint32_t)k, fw, fb);
+  launch(bn_fold_kernel, (unsigned)cdiv(total, 256), 256, 0, st(stream), w, bias, gamma, beta, rm, rv, eps, total, (uint32_t)k, fw, fb);
   return check_launch("bn_fold");
 }
 
@@ -745,7 +756,7 @@ int omt_bn_backward_add(const OmtAct* gy, const OmtAct* x, const OmtAct* y, cons
   const uint32_t* bits = (relu && (flags & OMT_BN_MASKBITS)) ? reinterpret_cast<const uint32_t*>(y->p + (int64_t)n * c * h * w) : nullptr;
   r = launch_part<1>(lay, x->p, gy->p, relu ? y->p : x->p, bits, mean, invstd, relu, n, c, h, w, &S, part, s);
   if (r) return r;
-  bn_bwd_fin<<<(unsigned)cdiv((int64_t)c * 32, 256), 256, 0, s>>>(part, c, S, scale, dgb, raw);
+  launch(bn_bwd_fin, (unsigned)cdiv((int64_t)c * 32, 256), 256, 0, s, part, c, S, scale, dgb, raw);
   r = check_launch("bn_bwd_fin");
   if (r || !dx || !dx->p) return r;
   BnEw a{};

@@ -83,6 +83,7 @@ struct CallTimer {
 };
 
 __global__ void __launch_bounds__(256) scale_copy_kernel(float* __restrict__ dst, const float* __restrict__ src, int64_t n, float scale) {
+  pdl_wait();
   int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i + 3 < n) {
     float4 v = __ldg(reinterpret_cast<const float4*>(src + i));
@@ -92,6 +93,7 @@ __global__ void __launch_bounds__(256) scale_copy_kernel(float* __restrict__ dst
   }
 }
 __global__ void __launch_bounds__(256) scale_copy_scalar_kernel(float* __restrict__ dst, const float* __restrict__ src, int64_t n, float scale) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dst[i] = src[i] * scale;
 }
@@ -100,6 +102,7 @@ __global__ void __launch_bounds__(256) scale_copy_scalar_kernel(float* __restric
 // destination's. View both tensors as [n][c][hw]; one of (c, hw) is contiguous in each.
 __global__ void __launch_bounds__(256) transpose_kernel(const float* __restrict__ src, float* __restrict__ dst, int c, int hw,
                                                         bool src_c_fast) {
+  pdl_wait();
   __shared__ float tile[32][33];
   const int img = blockIdx.z;
   const int c0 = blockIdx.y * 32, p0 = blockIdx.x * 32;
@@ -128,6 +131,7 @@ __global__ void __launch_bounds__(256) transpose_kernel(const float* __restrict_
   }
 }
 __global__ void __launch_bounds__(256) strided_copy_kernel(ActView src, ActView dst, int n, int c, int h, int w) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)n * c * h * w) return;
   int x = (int)(i % w); i /= w;
@@ -176,6 +180,7 @@ namespace omt {
 constexpr size_t TAPS_MAX_BYTES = (size_t)1 << 30;  // beyond this T the CUDA-core kernel runs instead
 
 __global__ void __launch_bounds__(256) taps_weight_kernel(const float* __restrict__ w, float* __restrict__ wm, int co, int ci, int kk, int colsp) {
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;  // wm[o][t * ci + c] = w[o][c][t]; columns past ci * kk are zero
   if (i >= co * colsp) return;
   const int o = i / colsp, col = i - o * colsp;
@@ -191,6 +196,7 @@ struct Col2imArgs {
 // one thread per input pixel (consecutive threads, consecutive x): the s threads of one stride period read s * ci consecutive
 // floats of one row of T per tap
 __global__ void __launch_bounds__(256) col2im_kernel(Col2imArgs a) {
+  pdl_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)a.n * a.ih * a.iw) return;
   const int x = (int)(i % a.iw);
@@ -238,14 +244,14 @@ static int dgrad_by_taps(const OmtConvGeo* g, const OmtAct* gy, const float* w, 
   float* wm = (float*)sc.p;
   float* T = wm + wm_floats;
   cudaStream_t s = st(stream);
-  taps_weight_kernel<<<(unsigned)cdiv((int64_t)g->co * colsp, 256), 256, 0, s>>>(w, wm, g->co, g->ci, kk, colsp);
+  launch(taps_weight_kernel, (unsigned)cdiv((int64_t)g->co * colsp, 256), 256, 0, s, w, wm, g->co, g->ci, kk, colsp);
   r = check_launch("conv_dgrad_taps_weights");
   if (r) return r;
   OmtAct t{T, (int64_t)colsp * g->oh * g->ow, 1, (int64_t)colsp * g->ow, colsp};
   r = tc_conv_dgrad(&g1, gy, wm, &t, 0, ws.p, s);
   if (r) return r;
   Col2imArgs a{T, view(dx), g->n, g->ci, g->ih, g->iw, g->oh, g->ow, g->ks, g->stride, g->pad, colsp};
-  col2im_kernel<<<(unsigned)cdiv((int64_t)g->n * g->ih * g->iw, 256), 256, 0, s>>>(a);
+  launch(col2im_kernel, (unsigned)cdiv((int64_t)g->n * g->ih * g->iw, 256), 256, 0, s, a);
   return check_launch("conv_dgrad_col2im");
 }
 }  // namespace omt
@@ -436,9 +442,9 @@ int omt_scale_copy(float* dst, const float* src, int64_t n, float scale, omt_str
   OMT_REQUIRE(dst && src && n >= 0, "omt_scale_copy: bad arguments");
   if (n == 0) return OMT_OK;
   if (((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0)
-    scale_copy_kernel<<<(unsigned)cdiv(cdiv(n, 4), 256), 256, 0, st(stream)>>>(dst, src, n, scale);
+    launch(scale_copy_kernel, (unsigned)cdiv(cdiv(n, 4), 256), 256, 0, st(stream), dst, src, n, scale);
   else
-    scale_copy_scalar_kernel<<<(unsigned)cdiv(n, 256), 256, 0, st(stream)>>>(dst, src, n, scale);
+    launch(scale_copy_scalar_kernel, (unsigned)cdiv(n, 256), 256, 0, st(stream), dst, src, n, scale);
   return check_launch("scale_copy");
 }
 
@@ -449,10 +455,10 @@ int omt_act_copy(const OmtAct* src, const OmtAct* dst, int32_t n, int32_t c, int
   if ((s_nchw && d_nchw) || (s_nhwc && d_nhwc)) return omt_memcpy_d2d(dst->p, src->p, total * sizeof(float), stream);
   if (((s_nchw && d_nhwc) || (s_nhwc && d_nchw)) && n <= 65535) {
     dim3 grid((unsigned)cdiv(h * w, 32), (unsigned)cdiv(c, 32), n);
-    transpose_kernel<<<grid, 256, 0, st(stream)>>>(src->p, dst->p, c, h * w, s_nhwc);
+    launch(transpose_kernel, grid, 256, 0, st(stream), src->p, dst->p, c, h * w, s_nhwc);
     return check_launch("act_transpose");
   }
-  strided_copy_kernel<<<(unsigned)cdiv(total, 256), 256, 0, st(stream)>>>(view(src), view(dst), n, c, h, w);
+  launch(strided_copy_kernel, (unsigned)cdiv(total, 256), 256, 0, st(stream), view(src), view(dst), n, c, h, w);
   return check_launch("act_strided_copy");
 }
 

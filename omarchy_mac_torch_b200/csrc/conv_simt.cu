@@ -220,6 +220,7 @@ struct Wgrad {
 // BN/2 apart, threads m-fastest so stores along m coalesce for NCHW outputs.
 template <class L, int BM, int BN, int TM, int TN>
 __global__ void __launch_bounds__(256) conv_gemm_simt(ConvArgs g) {
+  pdl_wait();
   constexpr int TY = BM / TM, GM = TM / 4, GN = TN / 4;
   constexpr int RA = BM / 32, RB = (BN + 31) / 32;
   static_assert((BM / TM) * (BN / TN) == 256, "256 threads");
@@ -314,6 +315,7 @@ __global__ void __launch_bounds__(256) conv_gemm_simt(ConvArgs g) {
 // dw[i] = scale * sum_z part[z][i]   (reference csrc/kernels/gemm_reduce.wgsl:7-13, vectorised)
 __global__ void __launch_bounds__(256) slab_sum_kernel(const float* __restrict__ part, float* __restrict__ out, int64_t total,
                                                        int slices, float scale) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   float s = 0.f;
@@ -330,18 +332,18 @@ static int launch_gemm(const ConvArgs& a, int64_t Mmax, int64_t N, int gz, cudaS
   OMT_REQUIRE(cdiv(N, N <= 16 ? 16 : 64) <= 65535 && gz <= 65535, "%s: %lld GEMM columns exceed the launch grid", name, (long long)N);
   if (N <= 16) {
     dim3 grid((unsigned)cdiv(Mmax, 256), (unsigned)cdiv(N, 16), gz);
-    conv_gemm_simt<L, 256, 16, 4, 4><<<grid, 256, 0, s>>>(a);
+    launch(conv_gemm_simt<L, 256, 16, 4, 4>, grid, 256, 0, s, a);
   } else if (N <= 64 || blocks(128, 128) < sms) {
     if (blocks(128, 64) < sms) {
       dim3 grid((unsigned)cdiv(Mmax, 64), (unsigned)cdiv(N, 64), gz);
-      conv_gemm_simt<L, 64, 64, 4, 4><<<grid, 256, 0, s>>>(a);
+      launch(conv_gemm_simt<L, 64, 64, 4, 4>, grid, 256, 0, s, a);
     } else {
       dim3 grid((unsigned)cdiv(Mmax, 128), (unsigned)cdiv(N, 64), gz);
-      conv_gemm_simt<L, 128, 64, 8, 4><<<grid, 256, 0, s>>>(a);
+      launch(conv_gemm_simt<L, 128, 64, 8, 4>, grid, 256, 0, s, a);
     }
   } else {
     dim3 grid((unsigned)cdiv(Mmax, 128), (unsigned)cdiv(N, 128), gz);
-    conv_gemm_simt<L, 128, 128, 8, 8><<<grid, 256, 0, s>>>(a);
+    launch(conv_gemm_simt<L, 128, 128, 8, 8>, grid, 256, 0, s, a);
   }
   return check_launch(name);
 }
@@ -376,6 +378,7 @@ struct DgSmallArgs {
 };
 
 __global__ void __launch_bounds__(128) dgrad_small_ci_kernel(DgSmallArgs a) {
+  pdl_wait();
   extern __shared__ float4 wsm[];  // [jy * jx][co]
   const int s = a.stride;
   const int py = blockIdx.y / s, px = blockIdx.y - py * s, img = blockIdx.z;
@@ -450,7 +453,7 @@ int dgrad_small_ci(const OmtConvGeo* g, const OmtAct* gy, const float* w, const 
   }
   const int64_t per_phase = cdiv(g->ih, g->stride) * cdiv(g->iw, g->stride);
   dim3 grid((unsigned)cdiv(per_phase, 128), (unsigned)(g->stride * g->stride), (unsigned)g->n);
-  dgrad_small_ci_kernel<<<grid, 128, smem, s>>>(a);
+  launch(dgrad_small_ci_kernel, grid, 128, smem, s, a);
   return check_launch("conv_dgrad_small_ci");
 }
 
@@ -488,7 +491,7 @@ int simt_conv_wgrad(const OmtConvGeo* g, const OmtAct* x, const OmtAct* gy, floa
   int r = launch_gemm<Wgrad>(a, a.M, a.N, a.slices, s, "conv_wgrad_simt");
   if (r != OMT_OK || a.slices == 1) return r;
   int64_t total = (int64_t)a.M * a.N;
-  slab_sum_kernel<<<(unsigned)cdiv(total, 256), 256, 0, s>>>(part, dw, total, a.slices, scale);
+  launch(slab_sum_kernel, (unsigned)cdiv(total, 256), 256, 0, s, part, dw, total, a.slices, scale);
   return check_launch("conv_wgrad_slab_sum");
 }
 
@@ -546,6 +549,7 @@ namespace omt {
 // One block per (channel, slice) with 128-bit loads when the plane is contiguous, then a second tiny kernel; the
 // reference used one workgroup per channel (csrc/kernels/csum_nchw.wgsl), i.e. 64 blocks for 64 channels.
 __global__ void __launch_bounds__(256) csum_part_kernel(ActView gy, int n, int c, int h, int w, int S, float* part) {
+  pdl_wait();
   __shared__ float red[32];
   int ch = blockIdx.x, sl = blockIdx.y;
   int hw = h * w;
@@ -571,6 +575,7 @@ __global__ void __launch_bounds__(256) csum_part_kernel(ActView gy, int n, int c
   if (threadIdx.x == 0) part[ch * S + sl] = s;
 }
 __global__ void csum_fin_kernel(const float* part, int c, int S, float scale, float* out) {
+  pdl_wait();
   int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
   float s = 0.f;
@@ -580,6 +585,7 @@ __global__ void csum_fin_kernel(const float* part, int c, int S, float scale, fl
 // channels-last: threads across channels, blocks across pixel ranges, atomics avoided by a two-level sum
 __global__ void __launch_bounds__(256) csum_nhwc_part_kernel(const float* __restrict__ gy, int64_t pixels, int c, int S,
                                                              float* part) {
+  pdl_wait();
   int ch = blockIdx.x * blockDim.x + threadIdx.x, sl = blockIdx.y;
   if (ch >= c) return;
   float s = 0.f;
@@ -604,14 +610,14 @@ extern "C" int omt_conv_bias_grad(const OmtAct* gy, int32_t n, int32_t c, int32_
   float* part = (float*)sc.p;
   if (nhwc) {
     dim3 grid((unsigned)cdiv(c, 256), S);
-    csum_nhwc_part_kernel<<<grid, 256, 0, s>>>(gy->p, (int64_t)n * h * w, c, S, part);
+    launch(csum_nhwc_part_kernel, grid, 256, 0, s, gy->p, (int64_t)n * h * w, c, S, part);
     r = check_launch("bias_grad_nhwc_part");
   } else {
     dim3 grid(c, S);
-    csum_part_kernel<<<grid, 256, 0, s>>>(view(gy), n, c, h, w, S, part);
+    launch(csum_part_kernel, grid, 256, 0, s, view(gy), n, c, h, w, S, part);
     r = check_launch("bias_grad_part");
   }
   if (r) return r;
-  csum_fin_kernel<<<(unsigned)cdiv(c, 128), 128, 0, s>>>(part, c, S, scale, db);
+  launch(csum_fin_kernel, (unsigned)cdiv(c, 128), 128, 0, s, part, c, S, scale, db);
   return check_launch("bias_grad_fin");
 }

@@ -495,6 +495,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if constexpr (PAIR) cluster_sync_all();  // the other CTA's barriers are initialised before anything here signals them
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();  // everything above touches only this CTA: it overlaps the end of the kernel in front
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -890,6 +891,7 @@ struct SplitArgs {
   int window;  // forward, window mode: tap = filter row ky, column k' = kx*4 + c
 };
 __global__ void __launch_bounds__(256) weight_split_kernel(const float* __restrict__ w, float* __restrict__ out, SplitArgs a) {
+  pdl_wait();
   const int rows = a.dgrad ? a.ci : a.co, chans = a.window ? a.cpad : (a.dgrad ? a.co : a.ci), kk = a.kh * a.kw;
   const int64_t total = (int64_t)rows * kk * a.cpad;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -972,6 +974,7 @@ int plan_splits(int64_t M, int64_t N, int kblocks, int bn) {
 
 // y(m, n) = epilogue(sum over splits of part[s][m][n]) for the GEMM row m = (img, oy, ox) of the (sub-)convolution
 __global__ void __launch_bounds__(256) splitk_epilogue_kernel(TcArgs g) {
+  pdl_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)g.M * g.N) return;
   const int n = (int)(i % g.N);
@@ -1048,10 +1051,10 @@ static int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_w, const
   using SP = Smem<BN, ACC1, true>;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2u * (unsigned)clusters); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = SP::TOTAL; cfg.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = 2; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-  cfg.attrs = &at; cfg.numAttrs = 1;
+  cudaLaunchAttribute at[2] = {{}, pdl_attr()};
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = 2;
   OMT_CUDA(cudaLaunchKernelEx(&cfg, conv_tc_kernel<BN, false, ACC1, true>, map_a, map_w, map_y, a));
   return check_launch(BN == 64 ? "conv_tc_256x64_pair" : (BN == 128 ? "conv_tc_256x128_pair" : (ACC1 ? "conv_tc_256x256_pair_acc1" : "conv_tc_256x256_pair")));
 }
@@ -1132,13 +1135,13 @@ int launch_tc(const TcProblem& p, const float* wsplit, const TcArgs& args, int s
     return acc1 ? launch_pair<256, true>(map_a, map_w, map_y, a, std::min(work, clusters), s)
                 : launch_pair<256, false>(map_a, map_w, map_y, a, std::min(work, clusters), s);
   }
-  if (splits > 1) conv_tc_kernel<BN, true><<<grid, TC_THREADS, S::TOTAL, s>>>(map_a, map_w, map_y, a);
-  else if (acc1) conv_tc_kernel<BN, false, BN == 256><<<grid, TC_THREADS, S::TOTAL, s>>>(map_a, map_w, map_y, a);
-  else if (BN == 64 && a_tmem_enabled()) conv_tc_kernel<BN, false, false, false, BN == 64><<<grid, TC_THREADS, S::TOTAL, s>>>(map_a, map_w, map_y, a);
-  else conv_tc_kernel<BN, false><<<grid, TC_THREADS, S::TOTAL, s>>>(map_a, map_w, map_y, a);
+  if (splits > 1) launch(conv_tc_kernel<BN, true>, grid, TC_THREADS, S::TOTAL, s, map_a, map_w, map_y, a);
+  else if (acc1) launch(conv_tc_kernel<BN, false, BN == 256>, grid, TC_THREADS, S::TOTAL, s, map_a, map_w, map_y, a);
+  else if (BN == 64 && a_tmem_enabled()) launch(conv_tc_kernel<BN, false, false, false, BN == 64>, grid, TC_THREADS, S::TOTAL, s, map_a, map_w, map_y, a);
+  else launch(conv_tc_kernel<BN, false>, grid, TC_THREADS, S::TOTAL, s, map_a, map_w, map_y, a);
   int r = check_launch(BN == 64 ? (splits == 1 && a_tmem_enabled() ? "conv_tc_128x64_atmem" : "conv_tc_128x64") : (BN == 128 ? "conv_tc_128x128" : (acc1 ? "conv_tc_128x256_acc1" : "conv_tc_128x256")));
   if (r || splits == 1) return r;
-  splitk_epilogue_kernel<<<(unsigned)cdiv((int64_t)a.M * a.N, 256), 256, 0, s>>>(a);
+  launch(splitk_epilogue_kernel, (unsigned)cdiv((int64_t)a.M * a.N, 256), 256, 0, s, a);
   return check_launch("conv_tc_splitk_epilogue");
 }
 
@@ -1157,7 +1160,7 @@ int run_tc(const TcProblem& p, const float* w, SplitArgs sp, float* wsplit, floa
   const int cpad = a.cblocks * BKF;
   sp.kh = p.kh; sp.kw = p.kw; sp.cpad = cpad;
   const int64_t total = (int64_t)p.rows * p.kh * p.kw * cpad;
-  weight_split_kernel<<<(unsigned)cdiv(total, 256), 256, 0, s>>>(w, wsplit, sp);
+  launch(weight_split_kernel, (unsigned)cdiv(total, 256), 256, 0, s, w, wsplit, sp);
   int r = check_launch("conv_tc_weight_split");
   if (r) return r;
   const int bn = pick_bn(p);
@@ -1283,6 +1286,7 @@ wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
   if constexpr (PAIR) cluster_sync_all();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_acc = *tmem_slot;
+  pdl_wait();  // everything above touches only this CTA: it overlaps the end of the kernel in front
 
   if (warp == 0) {
     if (lane == 0) {
@@ -1486,6 +1490,7 @@ wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 template <int SL>
 __global__ void __launch_bounds__(256) wgrad_tc_reduce_kernel(const float* __restrict__ part, float* __restrict__ dw, int co, int ci, int kk,
                                                               int cpad, int slices, float scale, int win_ks, int win_kb) {
+  pdl_wait();
   // threads run over (o, tap, c) with c fastest: the slab reads coalesce; the strided writes are 1/slices of the traffic
   constexpr int OUTS = 256 / SL;
   const int local = threadIdx.x % OUTS, sl = threadIdx.x / OUTS;
@@ -1523,8 +1528,8 @@ void launch_wgrad_reduce(const float* part, float* dw, int co, int ci, int kk, i
   const int64_t total = (int64_t)co * ci * kk;
   // (measured per ResNet-50 layer at batch 256: sharing an output among threads pays only for the one-tile layers with a slice
   // per SM, 64 -> 64 1x1 0.148 -> 0.135 ms; with 2-37 slices the plain kernel is as fast or faster)
-  if (slices >= 64) wgrad_tc_reduce_kernel<16><<<(unsigned)cdiv(total, 16), 256, 0, s>>>(part, dw, co, ci, kk, cpad, slices, scale, win_ks, win_kb);
-  else wgrad_tc_reduce_kernel<1><<<(unsigned)cdiv(total, 256), 256, 0, s>>>(part, dw, co, ci, kk, cpad, slices, scale, win_ks, win_kb);
+  if (slices >= 64) launch(wgrad_tc_reduce_kernel<16>, (unsigned)cdiv(total, 16), 256, 0, s, part, dw, co, ci, kk, cpad, slices, scale, win_ks, win_kb);
+  else launch(wgrad_tc_reduce_kernel<1>, (unsigned)cdiv(total, 256), 256, 0, s, part, dw, co, ci, kk, cpad, slices, scale, win_ks, win_kb);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -1533,6 +1538,7 @@ void launch_wgrad_reduce(const float* part, float* dw, int co, int ci, int kk, i
 // xs[n][ih][ws][4] = x[n][c][h][w - pad] (zero outside, zero for c >= ci): a channels-last copy padded to 4 channels and
 // by `pad` zero pixels on the left (and enough on the right), so that the window rows need no horizontal bounds handling.
 __global__ void __launch_bounds__(256) stage_window_kernel(ActView x, float* __restrict__ xs, int n, int ci, int ih, int iw, int ws, int pad) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t total = (int64_t)n * ih * ws;
   if (i >= total) return;
@@ -1631,8 +1637,8 @@ int launch_window(const OmtConvGeo* g, const WinPlan& w, const float* xs, const 
   OMT_REQUIRE(!(a.flags & OMT_EPI_BNSTATS) || a.store_mode == 2, "OMT_EPI_BNSTATS needs a dense channels-last output");
   const int m_tiles = g->n * w.tiles_x * w.tiles_y, n_tiles = (int)cdiv(a.N, BN);
   const unsigned grid = (unsigned)std::min<int64_t>((int64_t)m_tiles * n_tiles, sm_count());
-  if (BN == 64 && a_tmem_enabled()) conv_tc_kernel<BN, false, false, false, BN == 64><<<grid, TC_THREADS, S::TOTAL, s>>>(map_a, map_w, map_y, a);
-  else conv_tc_kernel<BN, false><<<grid, TC_THREADS, S::TOTAL, s>>>(map_a, map_w, map_y, a);
+  if (BN == 64 && a_tmem_enabled()) launch(conv_tc_kernel<BN, false, false, false, BN == 64>, grid, TC_THREADS, S::TOTAL, s, map_a, map_w, map_y, a);
+  else launch(conv_tc_kernel<BN, false>, grid, TC_THREADS, S::TOTAL, s, map_a, map_w, map_y, a);
   return check_launch(BN == 64 ? "conv_tc_window_128x64" : (BN == 128 ? "conv_tc_window_128x128" : "conv_tc_window_128x256"));
 }
 
@@ -1642,7 +1648,7 @@ int run_window_fwd(const OmtConvGeo* g, const OmtAct* x, const float* w, const f
   float* xs = (float*)ws;
   float* wsplit = xs + ((wp.stage_floats + 63) / 64) * 64;
   const int64_t total = (int64_t)g->n * g->ih * wp.ws;
-  stage_window_kernel<<<(unsigned)cdiv(total, 256), 256, 0, s>>>(view(x), xs, g->n, g->ci, g->ih, g->iw, wp.ws, g->pad);
+  launch(stage_window_kernel, (unsigned)cdiv(total, 256), 256, 0, s, view(x), xs, g->n, g->ci, g->ih, g->iw, wp.ws, g->pad);
   int r = check_launch("conv_tc_stage_window");
   if (r) return r;
   TcArgs a{};
@@ -1654,7 +1660,7 @@ int run_window_fwd(const OmtConvGeo* g, const OmtAct* x, const float* w, const f
   a.win_w = wp.win_w; a.win_h = wp.win_h; a.tiles_x = wp.tiles_x; a.tiles_y = wp.tiles_y;
   SplitArgs sp{g->co, g->ci, g->ks, g->ks, 1, wp.kb * BKF, 0, 0, 0, 1, 1};
   const int64_t wtotal = (int64_t)g->co * g->ks * wp.kb * BKF;
-  weight_split_kernel<<<(unsigned)cdiv(wtotal, 256), 256, 0, s>>>(w, wsplit, sp);
+  launch(weight_split_kernel, (unsigned)cdiv(wtotal, 256), 256, 0, s, w, wsplit, sp);
   r = check_launch("conv_tc_weight_split");
   if (r) return r;
   const int bn = g->co <= 64 ? 64 : (g->co <= 128 ? 128 : 256);
@@ -1857,14 +1863,14 @@ int launch_wgrad(const OmtConvGeo* g, const WgPlan& w, const float* x, const flo
   if constexpr (PAIR) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = dim3(WG_THREADS); cfg.dynamicSmemBytes = S::TOTAL; cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = 2; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-    cfg.attrs = &at; cfg.numAttrs = 1;
+    cudaLaunchAttribute at[2] = {{}, pdl_attr()};
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 2;
     OMT_CUDA(cudaLaunchKernelEx(&cfg, wgrad_tc_kernel<BN, PB, true>, map_x, map_g, a));
     return check_launch(BN == 64 ? "wgrad_tc_256x64_pair" : (BN == 128 ? "wgrad_tc_256x128_pair" : (BN == 192 ? "wgrad_tc_256x192_pair" : "wgrad_tc_256x256_pair")));
   }
-  wgrad_tc_kernel<BN, PB><<<grid, WG_THREADS, S::TOTAL, s>>>(map_x, map_g, a);
+  launch(wgrad_tc_kernel<BN, PB>, grid, WG_THREADS, S::TOTAL, s, map_x, map_g, a);
   if (w.mode & 16) return check_launch(BN == 64 ? "wgrad_tc_128x64_tap_pairs" : (BN == 128 ? "wgrad_tc_128x128_tap_pairs" : (BN == 192 ? "wgrad_tc_128x192_tap_pairs" : "wgrad_tc_128x256_tap_pairs")));
   return check_launch(BN == 64 ? "wgrad_tc_128x64" : (BN == 128 ? "wgrad_tc_128x128" : (BN == 192 ? "wgrad_tc_128x192" : "wgrad_tc_128x256")));
 }
@@ -2019,7 +2025,7 @@ int tc_conv_wgrad(const OmtConvGeo* g, const OmtAct* x, const OmtAct* gy, float*
   if (w.mode & 8) {  // padded 4-channel copy of x, as in the forward window mode
     const WinPlan wp = plan_window(g);
     const int64_t total = (int64_t)g->n * g->ih * wp.ws;
-    stage_window_kernel<<<(unsigned)cdiv(total, 256), 256, 0, s>>>(view(x), (float*)ws, g->n, g->ci, g->ih, g->iw, wp.ws, g->pad);
+    launch(stage_window_kernel, (unsigned)cdiv(total, 256), 256, 0, s, view(x), (float*)ws, g->n, g->ci, g->ih, g->iw, wp.ws, g->pad);
     int r0 = check_launch("conv_tc_stage_window");
     if (r0) return r0;
     xin = (const float*)ws;

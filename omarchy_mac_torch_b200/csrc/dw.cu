@@ -44,6 +44,7 @@ __device__ __forceinline__ void decode(int64_t i, int c, int h, int w, int& img,
 
 template <bool NHWC>
 __global__ void __launch_bounds__(256) dw_fwd_kernel(DwArgs a) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)a.n * a.c * a.oh * a.ow) return;
   int img, ch, oy, ox;
@@ -68,6 +69,7 @@ __global__ void __launch_bounds__(256) dw_fwd_kernel(DwArgs a) {
 
 // channels-last, 4 channels per thread: 128-bit loads of x, weights re-laid as float4 per tap on the fly
 __global__ void __launch_bounds__(256) dw_fwd_nhwc4_kernel(DwArgs a) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int c4n = a.c / 4;
   if (i >= (int64_t)a.n * c4n * a.oh * a.ow) return;
@@ -103,6 +105,7 @@ __global__ void __launch_bounds__(256) dw_fwd_nhwc4_kernel(DwArgs a) {
 // input gradient as a gather: dx[y,x] = sum over taps with (y+p-ky) % s == 0 of gy[(y+p-ky)/s, (x+p-kx)/s] * w[ky,kx]
 template <bool NHWC>
 __global__ void __launch_bounds__(256) dw_dgrad_kernel(DwArgs a) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)a.n * a.c * a.ih * a.iw) return;
   int img, ch, yy, xx;
@@ -127,6 +130,7 @@ __global__ void __launch_bounds__(256) dw_dgrad_kernel(DwArgs a) {
 // weight gradient, NCHW: block (channel, slice) walks output pixels; thread keeps KS*KS partial sums in registers
 template <int KS>
 __global__ void __launch_bounds__(256) dw_wgrad_nchw_kernel(DwArgs a, int S, float* __restrict__ part) {
+  pdl_wait();
   __shared__ float red[32];
   const int ch = blockIdx.x, sl = blockIdx.y, ohw = a.oh * a.ow;
   float acc[KS * KS];
@@ -159,6 +163,7 @@ __global__ void __launch_bounds__(256) dw_wgrad_nchw_kernel(DwArgs a, int S, flo
 }
 // any kernel size: one tap per blockIdx.z (re-reads the activations ks*ks times; only used for ks not in {3,5,7})
 __global__ void __launch_bounds__(256) dw_wgrad_tap_kernel(DwArgs a, int S, float* __restrict__ part) {
+  pdl_wait();
   __shared__ float red[32];
   const int ch = blockIdx.x, sl = blockIdx.y, t = blockIdx.z, ky = t / a.ks, kx = t - ky * a.ks, ohw = a.oh * a.ow;
   float acc = 0.f;
@@ -178,6 +183,7 @@ __global__ void __launch_bounds__(256) dw_wgrad_tap_kernel(DwArgs a, int S, floa
 // channels-last: one thread per channel (coalesced across c), slices over pixels; no block reduction needed
 template <int KS>
 __global__ void __launch_bounds__(128) dw_wgrad_nhwc_kernel(DwArgs a, int S, float* __restrict__ part) {
+  pdl_wait();
   const int ch = blockIdx.x * blockDim.x + threadIdx.x, sl = blockIdx.y;
   if (ch >= a.c) return;
   float acc[KS * KS];
@@ -210,6 +216,7 @@ __global__ void __launch_bounds__(128) dw_wgrad_nhwc_kernel(DwArgs a, int S, flo
 // the filter re-laid once per call as wt[tap][c] so a thread's four weights of a tap are one 128-bit load.
 // ---------------------------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) dw_weight_tc_kernel(const float* __restrict__ w, float* __restrict__ wt, int c, int kk) {
+  pdl_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x;  // i = t * c + ch
   if (i >= c * kk) return;
   int t = i / c, ch = i - t * c;
@@ -221,6 +228,7 @@ __global__ void __launch_bounds__(256) dw_weight_tc_kernel(const float* __restri
 // (TX-1)*stride + KS input pixels once and slides the taps over them in registers.
 template <int KS, int STRIDE, bool FLIP, int TX>
 __global__ void __launch_bounds__(256) dw_rows_nhwc4_kernel(DwArgs a, const float* __restrict__ wt) {
+  pdl_wait();
   constexpr int SPAN = (TX - 1) * STRIDE + KS;
   const int c4n = a.c >> 2, gx = (a.ow + TX - 1) / TX;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -279,6 +287,7 @@ __global__ void __launch_bounds__(256) dw_rows_nhwc4_kernel(DwArgs a, const floa
 
 // strided input gradient, channels-last: the gather of dw_dgrad_kernel on 4 channels at a time
 __global__ void __launch_bounds__(256) dw_dgrad_nhwc4_kernel(DwArgs a, const float* __restrict__ wt) {
+  pdl_wait();
   const int c4n = a.c >> 2;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)a.n * a.ih * a.iw * c4n) return;
@@ -308,6 +317,7 @@ __global__ void __launch_bounds__(256) dw_dgrad_nhwc4_kernel(DwArgs a, const flo
 // every tap takes its 4 products from registers.
 template <int KS, int STRIDE>
 __global__ void __launch_bounds__(256) dw_wgrad_nhwc4_kernel(DwArgs a, int S, int CL, float* __restrict__ part) {
+  pdl_wait();
   constexpr int TX = 4, SPAN = (TX - 1) * STRIDE + KS;
   extern __shared__ float4 red4[];  // [PL][CL]
   const int PL = blockDim.x / CL;
@@ -382,6 +392,7 @@ __global__ void __launch_bounds__(256) dw_wgrad_nhwc4_kernel(DwArgs a, int S, in
 }
 // one warp per output (ch, tap): lanes stride over the S slices, then a shuffle tree (fixed order: deterministic)
 __global__ void __launch_bounds__(256) dw_wgrad_fin_kernel(const float* __restrict__ part, int64_t total, int kk, int S, float scale, float* out) {
+  pdl_wait();
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // i = ch*kk + t
   const int lane = threadIdx.x & 31;
   if (i >= total) return;
@@ -508,6 +519,7 @@ constexpr size_t ring_bytes() { return (size_t)ROLL_DEPTH * SPAN * ROLL_THREADS 
 // Forward (FLIP = false) and stride-1 input gradient (FLIP = true: taps mirrored, pad = ks-1-pad, the caller swaps the tensors).
 template <int KS, int S, bool FLIP, int TX, int CH, bool WREG>
 __global__ void __launch_bounds__(ROLL_THREADS) dw_roll_kernel(DwArgs a, const float* __restrict__ wt, int seg_rows, int segs) {
+  pdl_wait();
   constexpr int SPAN = (TX - 1) * S + KS, R = (KS + S - 1) / S, U = R * S;
   extern __shared__ __align__(16) uint8_t ring_raw[];
   const int cqn = a.c / CH, gx = (a.ow + TX - 1) / TX;
@@ -650,6 +662,7 @@ __global__ void __launch_bounds__(ROLL_THREADS) dw_roll_kernel(DwArgs a, const f
 // the parity of the strip's first column, so no division or modulo is left per tap.
 template <int KS, int TX, int CH>
 __global__ void __launch_bounds__(256) dw_dgrad_s2_kernel(DwArgs a, const float* __restrict__ wt) {  // a.x = gy, a.y = dx
+  pdl_wait();
   constexpr int HALF = (KS - 1) / 2, G = HALF + TX / 2 + 1;
   const int cqn = a.c / CH, gx = (a.iw + TX - 1) / TX;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -698,6 +711,7 @@ __global__ void __launch_bounds__(256) dw_dgrad_s2_kernel(DwArgs a, const float*
 // whole walk. Pixel lanes are summed through shared memory in a fixed order, slices (blockIdx.y) by dw_wgrad_fin_kernel.
 template <int KS, int S, int TX, int CH>
 __global__ void __launch_bounds__(ROLL_THREADS) dw_wgrad_roll_kernel(DwArgs a, int SL, int CL, int seg_rows, int segs, float* __restrict__ part) {
+  pdl_wait();
   constexpr int SPAN = (TX - 1) * S + KS, R = (KS + S - 1) / S, U = R * S;
   extern __shared__ __align__(16) uint8_t ring_raw[];  // the row ring; after the walk its start is reused as [PL][CL] vectors of CH floats
   const int PL = blockDim.x / CL;
@@ -849,13 +863,13 @@ static void launch_roll(const DwArgs& a, const float* wt, cudaStream_t s) {
   const int rows = strip_rows(a.oh, KS, per_seg, (int64_t)sm_count() * 1536, segs);
   constexpr size_t smem = ring_bytes<CH, SPAN>();
   allow_shared_memory<dw_roll_kernel<KS, S, FLIP, TX, CH, WREG>>(smem);
-  dw_roll_kernel<KS, S, FLIP, TX, CH, WREG><<<(unsigned)cdiv(per_seg * segs, ROLL_THREADS), ROLL_THREADS, smem, s>>>(a, wt, rows, segs);
+  launch(dw_roll_kernel<KS, S, FLIP, TX, CH, WREG>, (unsigned)cdiv(per_seg * segs, ROLL_THREADS), ROLL_THREADS, smem, s, a, wt, rows, segs);
 }
 template <int KS, int S, int TX, int CH>
 static void launch_wgrad_roll(const DwArgs& a, dim3 grid, int SL, int CL, int rows, int segs, float* part, cudaStream_t s) {
   constexpr size_t smem = ring_bytes<CH, (TX - 1) * S + KS>();
   allow_shared_memory<dw_wgrad_roll_kernel<KS, S, TX, CH>>(smem);
-  dw_wgrad_roll_kernel<KS, S, TX, CH><<<grid, ROLL_THREADS, smem, s>>>(a, SL, CL, rows, segs, part);
+  launch(dw_wgrad_roll_kernel<KS, S, TX, CH>, grid, ROLL_THREADS, smem, s, a, SL, CL, rows, segs, part);
 }
 // Which kernel serves which case (measured on 128 x 96 x 56 x 56 and 64 x 96 x 112 x 112 -> 56 x 56, fraction of the copy
 // bandwidth): stride 1, 3x3 and 5x5: the rolling kernel (3x3: 0.75 against 0.66); stride 2 and 7x7: one output row per thread
@@ -865,13 +879,13 @@ static void launch_rows_ks(const DwArgs& a, int stride, const float* wt, cudaStr
   if (stride == 1 && KS <= 5) return launch_roll<KS == 7 ? 5 : KS, 1, FLIP>(a, wt, s);
   const int64_t total = (int64_t)a.n * a.oh * cdiv(a.ow, 4) * (a.c / 4);
   const unsigned blocks = (unsigned)cdiv(total, 256);
-  if (stride == 1) dw_rows_nhwc4_kernel<KS, 1, FLIP, 4><<<blocks, 256, 0, s>>>(a, wt);
-  else dw_rows_nhwc4_kernel<KS, 2, FLIP, 4><<<blocks, 256, 0, s>>>(a, wt);
+  if (stride == 1) launch(dw_rows_nhwc4_kernel<KS, 1, FLIP, 4>, blocks, 256, 0, s, a, wt);
+  else launch(dw_rows_nhwc4_kernel<KS, 2, FLIP, 4>, blocks, 256, 0, s, a, wt);
 }
 // `a` describes the convolution the kernel performs (for the flipped input gradient: gy -> dx with stride 1)
 static int launch_rows(const DwArgs& a, const OmtConvGeo* g, float* wt, bool flip, cudaStream_t s, const char* name) {
   const int kk = g->ks * g->ks;
-  dw_weight_tc_kernel<<<(unsigned)cdiv((int64_t)a.c * kk, 256), 256, 0, s>>>(a.w, wt, a.c, kk);
+  launch(dw_weight_tc_kernel, (unsigned)cdiv((int64_t)a.c * kk, 256), 256, 0, s, a.w, wt, a.c, kk);
   const int stride = flip ? 1 : g->stride;
   if (flip) {
     if (g->ks == 3) launch_rows_ks<3, true>(a, stride, wt, s);
@@ -906,11 +920,11 @@ int omt_dw_fwd(const OmtConvGeo* g, const OmtAct* x, const float* w, const float
       if (r) return r;
       return launch_rows(a, g, (float*)sc.p, false, st(stream), "dw_fwd_rows_nhwc4");
     }
-    dw_fwd_nhwc4_kernel<<<(unsigned)cdiv(total / 4, 256), 256, 0, st(stream)>>>(a);
+    launch(dw_fwd_nhwc4_kernel, (unsigned)cdiv(total / 4, 256), 256, 0, st(stream), a);
     return check_launch("dw_fwd_nhwc4");
   }
-  if (yn) dw_fwd_kernel<true><<<(unsigned)cdiv(total, 256), 256, 0, st(stream)>>>(a);
-  else dw_fwd_kernel<false><<<(unsigned)cdiv(total, 256), 256, 0, st(stream)>>>(a);
+  if (yn) launch(dw_fwd_kernel<true>, (unsigned)cdiv(total, 256), 256, 0, st(stream), a);
+  else launch(dw_fwd_kernel<false>, (unsigned)cdiv(total, 256), 256, 0, st(stream), a);
   return check_launch("dw_fwd");
 }
 
@@ -931,20 +945,20 @@ int omt_dw_dgrad(const OmtConvGeo* g, const OmtAct* gy, const float* w, const Om
       return launch_rows(f, g, (float*)sc.p, true, st(stream), "dw_dgrad_rows_nhwc4");
     }
     const int kk = g->ks * g->ks;
-    dw_weight_tc_kernel<<<(unsigned)cdiv((int64_t)g->ci * kk, 256), 256, 0, st(stream)>>>(w, (float*)sc.p, g->ci, kk);
+    launch(dw_weight_tc_kernel, (unsigned)cdiv((int64_t)g->ci * kk, 256), 256, 0, st(stream), w, (float*)sc.p, g->ci, kk);
     if (g->stride == 2 && rows_ok(g)) {
       const int64_t threads = (int64_t)g->n * g->ih * cdiv(g->iw, 4) * (g->ci / 4);
       const unsigned blocks = (unsigned)cdiv(threads, 256);
-      if (g->ks == 3) dw_dgrad_s2_kernel<3, 4, 4><<<blocks, 256, 0, st(stream)>>>(a, (const float*)sc.p);
-      else if (g->ks == 5) dw_dgrad_s2_kernel<5, 4, 4><<<blocks, 256, 0, st(stream)>>>(a, (const float*)sc.p);
-      else dw_dgrad_s2_kernel<7, 4, 4><<<blocks, 256, 0, st(stream)>>>(a, (const float*)sc.p);
+      if (g->ks == 3) launch(dw_dgrad_s2_kernel<3, 4, 4>, blocks, 256, 0, st(stream), a, (const float*)sc.p);
+      else if (g->ks == 5) launch(dw_dgrad_s2_kernel<5, 4, 4>, blocks, 256, 0, st(stream), a, (const float*)sc.p);
+      else launch(dw_dgrad_s2_kernel<7, 4, 4>, blocks, 256, 0, st(stream), a, (const float*)sc.p);
       return check_launch("dw_dgrad_s2_nhwc4");
     }
-    dw_dgrad_nhwc4_kernel<<<(unsigned)cdiv(total / 4, 256), 256, 0, st(stream)>>>(a, (const float*)sc.p);
+    launch(dw_dgrad_nhwc4_kernel, (unsigned)cdiv(total / 4, 256), 256, 0, st(stream), a, (const float*)sc.p);
     return check_launch("dw_dgrad_nhwc4");
   }
-  if (is_nhwc(dx, g->ci, g->ih, g->iw)) dw_dgrad_kernel<true><<<(unsigned)cdiv(total, 256), 256, 0, st(stream)>>>(a);
-  else dw_dgrad_kernel<false><<<(unsigned)cdiv(total, 256), 256, 0, st(stream)>>>(a);
+  if (is_nhwc(dx, g->ci, g->ih, g->iw)) launch(dw_dgrad_kernel<true>, (unsigned)cdiv(total, 256), 256, 0, st(stream), a);
+  else launch(dw_dgrad_kernel<false>, (unsigned)cdiv(total, 256), 256, 0, st(stream), a);
   return check_launch("dw_dgrad");
 }
 
@@ -991,13 +1005,13 @@ int omt_dw_wgrad(const OmtConvGeo* g, const OmtAct* x, const OmtAct* gy, float* 
       part = (float*)sc.p;
       dim3 grid(gx, S);
       const size_t smem = (size_t)PL * CL * sizeof(float4);
-      if (g->ks == 3) dw_wgrad_nhwc4_kernel<3, 2><<<grid, 256, smem, s>>>(a, S, CL, part);
-      else dw_wgrad_nhwc4_kernel<5, 2><<<grid, 256, smem, s>>>(a, S, CL, part);
+      if (g->ks == 3) launch(dw_wgrad_nhwc4_kernel<3, 2>, grid, 256, smem, s, a, S, CL, part);
+      else launch(dw_wgrad_nhwc4_kernel<5, 2>, grid, 256, smem, s, a, S, CL, part);
     }
     r = check_launch(g->stride == 1 ? "dw_wgrad_strips_nhwc" : "dw_wgrad_nhwc4");
     if (r) return r;
     const int64_t total = (int64_t)c * kk;
-    dw_wgrad_fin_kernel<<<(unsigned)cdiv(total * 32, 256), 256, 0, s>>>(part, total, kk, S, scale, dw);
+    launch(dw_wgrad_fin_kernel, (unsigned)cdiv(total * 32, 256), 256, 0, s, part, total, kk, S, scale, dw);
     return check_launch("dw_wgrad_fin");
   }
   int S;
@@ -1013,24 +1027,24 @@ int omt_dw_wgrad(const OmtConvGeo* g, const OmtAct* x, const OmtAct* gy, float* 
   float* part = (float*)sc.p;
   if (nhwc && reg) {
     dim3 grid((unsigned)cdiv(c, 128), S);
-    if (g->ks == 3) dw_wgrad_nhwc_kernel<3><<<grid, 128, 0, s>>>(a, S, part);
-    else if (g->ks == 5) dw_wgrad_nhwc_kernel<5><<<grid, 128, 0, s>>>(a, S, part);
-    else dw_wgrad_nhwc_kernel<7><<<grid, 128, 0, s>>>(a, S, part);
+    if (g->ks == 3) launch(dw_wgrad_nhwc_kernel<3>, grid, 128, 0, s, a, S, part);
+    else if (g->ks == 5) launch(dw_wgrad_nhwc_kernel<5>, grid, 128, 0, s, a, S, part);
+    else launch(dw_wgrad_nhwc_kernel<7>, grid, 128, 0, s, a, S, part);
     r = check_launch("dw_wgrad_nhwc");
   } else if (reg) {
     dim3 grid(c, S);
-    if (g->ks == 3) dw_wgrad_nchw_kernel<3><<<grid, 256, 0, s>>>(a, S, part);
-    else if (g->ks == 5) dw_wgrad_nchw_kernel<5><<<grid, 256, 0, s>>>(a, S, part);
-    else dw_wgrad_nchw_kernel<7><<<grid, 256, 0, s>>>(a, S, part);
+    if (g->ks == 3) launch(dw_wgrad_nchw_kernel<3>, grid, 256, 0, s, a, S, part);
+    else if (g->ks == 5) launch(dw_wgrad_nchw_kernel<5>, grid, 256, 0, s, a, S, part);
+    else launch(dw_wgrad_nchw_kernel<7>, grid, 256, 0, s, a, S, part);
     r = check_launch("dw_wgrad_nchw");
   } else {
     dim3 grid(c, S, kk);
-    dw_wgrad_tap_kernel<<<grid, 256, 0, s>>>(a, S, part);
+    launch(dw_wgrad_tap_kernel, grid, 256, 0, s, a, S, part);
     r = check_launch("dw_wgrad_tap");
   }
   if (r) return r;
   int64_t total = (int64_t)c * kk;
-  dw_wgrad_fin_kernel<<<(unsigned)cdiv(total * 32, 256), 256, 0, s>>>(part, total, kk, S, scale, dw);
+  launch(dw_wgrad_fin_kernel, (unsigned)cdiv(total * 32, 256), 256, 0, s, part, total, kk, S, scale, dw);
   return check_launch("dw_wgrad_fin");
 }
 

@@ -54,6 +54,7 @@ struct LossArgs {
 // SOFTMAX: x holds logits and logp is written; else x holds log-probabilities. NLL: the loss part runs.
 template <bool SOFTMAX, bool NLL>
 __global__ void __launch_bounds__(LOSS_WARPS * 32) loss_fwd_kernel(LossArgs a) {
+  pdl_wait();
   __shared__ float red[32];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -109,6 +110,7 @@ struct LossBwdArgs {
 
 // dx = g - exp(logp) * rowsum(g)
 __global__ void __launch_bounds__(LOSS_WARPS * 32) log_softmax_bwd_kernel(LossBwdArgs a) {
+  pdl_wait();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int64_t r = (int64_t)blockIdx.x * LOSS_WARPS + wid; r < a.rows; r += (int64_t)gridDim.x * LOSS_WARPS) {
     const float* gr = a.g + r * a.cols;
@@ -132,6 +134,7 @@ __device__ __forceinline__ float row_scale(const LossBwdArgs& a, int64_t r, int6
 // FUSED: dx = (exp(logp) - onehot(t)) * scale (gradient with respect to the logits); else dlogp = -onehot(t) * scale
 template <bool FUSED>
 __global__ void __launch_bounds__(LOSS_WARPS * 32) nll_bwd_kernel(LossBwdArgs a) {
+  pdl_wait();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int64_t r = (int64_t)blockIdx.x * LOSS_WARPS + wid; r < a.rows; r += (int64_t)gridDim.x * LOSS_WARPS) {
     const int64_t t = a.target[r];
@@ -170,7 +173,7 @@ static int nll_forward(const float* x, const int64_t* target, const float* weigh
     a.ticket = (unsigned int*)(a.row_w + rows);
     OMT_CUDA(cudaMemsetAsync(a.ticket, 0, sizeof(unsigned int), st(stream)));
   }
-  loss_fwd_kernel<SOFTMAX, true><<<loss_grid(rows), LOSS_WARPS * 32, 0, st(stream)>>>(a);
+  launch(loss_fwd_kernel<SOFTMAX, true>, loss_grid(rows), LOSS_WARPS * 32, 0, st(stream), a);
   return check_launch(name);
 }
 
@@ -185,7 +188,7 @@ int omt_log_softmax(const float* x, float* logp, int64_t rows, int32_t cols, omt
   if (int e = check_rows(rows, cols, "omt_log_softmax")) return e;
   LossArgs a{};
   a.x = x; a.logp = logp; a.rows = rows; a.cols = cols;
-  loss_fwd_kernel<true, false><<<loss_grid(rows), LOSS_WARPS * 32, 0, st(stream)>>>(a);
+  launch(loss_fwd_kernel<true, false>, loss_grid(rows), LOSS_WARPS * 32, 0, st(stream), a);
   return check_launch("log_softmax");
 }
 
@@ -194,7 +197,7 @@ int omt_log_softmax_backward(const float* g, const float* logp, float* dx, int64
   if (int e = check_rows(rows, cols, "omt_log_softmax_backward")) return e;
   LossBwdArgs a{};
   a.g = g; a.logp = logp; a.dx = dx; a.rows = rows; a.cols = cols;
-  log_softmax_bwd_kernel<<<loss_grid(rows), LOSS_WARPS * 32, 0, st(stream)>>>(a);
+  launch(log_softmax_bwd_kernel, loss_grid(rows), LOSS_WARPS * 32, 0, st(stream), a);
   return check_launch("log_softmax_bwd");
 }
 
@@ -217,8 +220,8 @@ static int nll_backward(bool fused, const float* g, const float* logp, const int
   LossBwdArgs a{};
   a.g = g; a.logp = logp; a.target = target; a.weight = weight; a.total_weight = total_weight; a.dx = dx;
   a.rows = rows; a.cols = cols; a.ignore = ignore; a.reduction = reduction;
-  if (fused) nll_bwd_kernel<true><<<loss_grid(rows), LOSS_WARPS * 32, 0, st(stream)>>>(a);
-  else nll_bwd_kernel<false><<<loss_grid(rows), LOSS_WARPS * 32, 0, st(stream)>>>(a);
+  if (fused) launch(nll_bwd_kernel<true>, loss_grid(rows), LOSS_WARPS * 32, 0, st(stream), a);
+  else launch(nll_bwd_kernel<false>, loss_grid(rows), LOSS_WARPS * 32, 0, st(stream), a);
   return check_launch(name);
 }
 

@@ -53,6 +53,7 @@ __device__ __forceinline__ void sgd_one(const SgdH& h, float& pv, float gr, floa
 }
 
 __global__ void __launch_bounds__(256) sgd_kernel(const DevParam* __restrict__ table, int count, SgdH h) {
+  pdl_wait();
   const int ti = find_tensor(table, count, blockIdx.x);
   const DevParam t = table[ti];
   const int64_t base = ((int64_t)blockIdx.x - t.first_chunk) * CHUNK;
@@ -97,6 +98,7 @@ __device__ __forceinline__ void adam_one(const AdamH& h, float bc1, float sbc2, 
 }
 
 __global__ void __launch_bounds__(256) adam_kernel(const DevParam* __restrict__ table, int count, AdamH h) {
+  pdl_wait();
   const int ti = find_tensor(table, count, blockIdx.x);
   const DevParam t = table[ti];
   const int64_t base = ((int64_t)blockIdx.x - t.first_chunk) * CHUNK;
@@ -203,7 +205,7 @@ int omt_sgd(const OmtParam* table, int32_t count, float lr, float momentum, floa
   int tensors = (int)(r >> 40);
   int64_t chunks = r & (((int64_t)1 << 40) - 1);
   SgdH h{lr, momentum, dampening, weight_decay, nesterov, first_step, maximize};
-  sgd_kernel<<<(unsigned)chunks, 256, 0, st(stream)>>>((const DevParam*)sc.p, tensors, h);
+  launch(sgd_kernel, (unsigned)chunks, 256, 0, st(stream), (const DevParam*)sc.p, tensors, h);
   return check_launch("sgd_multi");
 }
 
@@ -216,7 +218,7 @@ int omt_adam(const OmtParam* table, int32_t count, float lr, float beta1, float 
   int tensors = (int)(r >> 40);
   int64_t chunks = r & (((int64_t)1 << 40) - 1);
   AdamH h{lr, beta1, beta2, eps, weight_decay, decoupled, maximize};
-  adam_kernel<<<(unsigned)chunks, 256, 0, st(stream)>>>((const DevParam*)sc.p, tensors, h);
+  launch(adam_kernel, (unsigned)chunks, 256, 0, st(stream), (const DevParam*)sc.p, tensors, h);
   return check_launch("adam_multi");
 }
 

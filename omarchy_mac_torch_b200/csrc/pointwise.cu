@@ -77,6 +77,7 @@ __device__ __forceinline__ float pw_eval(int op, float a, float b, float c) {
 }
 
 __global__ void __launch_bounds__(PW_THREADS) pointwise_kernel(const __grid_constant__ PwArgs a) {
+  pdl_wait();
   __shared__ float val[PW_VALUES][PW_THREADS];
   const int tid = threadIdx.x;
   const int64_t i = (int64_t)blockIdx.x * PW_THREADS + tid;
@@ -178,6 +179,6 @@ extern "C" int omt_pointwise(const OmtPwProgram* prog, int32_t n_inputs, const f
     }
     if (same) a.same |= 1u << k;
   }
-  pointwise_kernel<<<(unsigned)cdiv(a.numel, PW_THREADS), PW_THREADS, 0, st(stream)>>>(a);
+  launch(pointwise_kernel, (unsigned)cdiv(a.numel, PW_THREADS), PW_THREADS, 0, st(stream), a);
   return check_launch("pointwise_program");
 }

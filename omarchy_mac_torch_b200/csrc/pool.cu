@@ -33,6 +33,7 @@ __device__ __forceinline__ void decode4(int64_t i, int c, int h, int w, int& img
 // ---- 2x2 stride-2 max pool with 2-bit argmax ----
 template <bool NHWC>
 __global__ void __launch_bounds__(256) pool2_fwd_kernel(ActView x, ActView y, uint8_t* idx, int n, int c, int oh, int ow) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)n * c * oh * ow) return;
   int img, ch, oy, ox;
@@ -50,6 +51,7 @@ __global__ void __launch_bounds__(256) pool2_fwd_kernel(ActView x, ActView y, ui
 template <bool NHWC>
 __global__ void __launch_bounds__(256) pool2_bwd_kernel(ActView g, const uint8_t* idx, ActView gx, int n, int c, int h, int w,
                                                         int oh, int ow) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)n * c * h * w) return;
   int img, ch, yy, xx;
@@ -64,6 +66,7 @@ __global__ void __launch_bounds__(256) pool2_bwd_kernel(ActView g, const uint8_t
 }
 template <bool NHWC>
 __global__ void __launch_bounds__(256) avgpool2_fwd_kernel(ActView x, ActView y, int n, int c, int oh, int ow) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)n * c * oh * ow) return;
   int img, ch, oy, ox;
@@ -73,6 +76,7 @@ __global__ void __launch_bounds__(256) avgpool2_fwd_kernel(ActView x, ActView y,
 }
 template <bool NHWC>
 __global__ void __launch_bounds__(256) avgpool2_bwd_kernel(ActView g, ActView gx, int n, int c, int h, int w, int oh, int ow) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)n * c * h * w) return;
   int img, ch, yy, xx;
@@ -92,6 +96,7 @@ __device__ __forceinline__ bool isnan_bits(float v) { return (__float_as_uint(v)
 
 template <bool NHWC>
 __global__ void __launch_bounds__(256) maxpool_fwd_kernel(PoolArgs a, int64_t* idx) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)a.n * a.c * a.oh * a.ow) return;
   int img, ch, oy, ox;
@@ -120,6 +125,7 @@ __global__ void __launch_bounds__(256) maxpool_fwd_kernel(PoolArgs a, int64_t* i
 }
 template <bool NHWC>
 __global__ void __launch_bounds__(256) maxpool_bwd_kernel(PoolArgs a, const int64_t* idx) {
+  pdl_wait();
   // a.x = gy (strides of the forward output), a.y = gx
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)a.n * a.c * a.ih * a.iw) return;
@@ -141,6 +147,7 @@ __global__ void __launch_bounds__(256) maxpool_bwd_kernel(PoolArgs a, const int6
 // Channels-last, 4 channels per thread (c % 4 == 0, dense tensors): 128-bit loads and stores, two 128-bit index accesses.
 // x / gx are [n, ih, iw, c], y / gy / idx are [n, oh, ow, c].
 __global__ void __launch_bounds__(256) maxpool_fwd_nhwc4_kernel(PoolArgs a, int64_t* __restrict__ idx) {
+  pdl_wait();
   const int c4 = a.c >> 2;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)a.n * a.oh * a.ow * c4) return;
@@ -175,6 +182,7 @@ __global__ void __launch_bounds__(256) maxpool_fwd_nhwc4_kernel(PoolArgs a, int6
   ip[1] = make_longlong2(bi[2], bi[3]);
 }
 __global__ void __launch_bounds__(256) maxpool_bwd_nhwc4_kernel(PoolArgs a, const int64_t* __restrict__ idx) {
+  pdl_wait();
   // a.x = gy, a.y = gx
   const int c4 = a.c >> 2;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -205,6 +213,7 @@ __global__ void __launch_bounds__(256) maxpool_bwd_nhwc4_kernel(PoolArgs a, cons
 // shifts and the loops unroll. Same update rule as above (first maximum wins, the first NaN wins outright).
 template <int KS, int ST, int TX>
 __global__ void __launch_bounds__(256) maxpool_fwd_nhwc4_fixed_kernel(PoolArgs a, int64_t* __restrict__ idx) {
+  pdl_wait();
   constexpr int SPAN = (TX - 1) * ST + KS;
   const int c4 = a.c >> 2, gx = (a.ow + TX - 1) / TX;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -272,6 +281,7 @@ __global__ void __launch_bounds__(256) maxpool_fwd_nhwc4_fixed_kernel(PoolArgs a
 }
 template <int KS, int ST>
 __global__ void __launch_bounds__(256) maxpool_bwd_nhwc4_fixed_kernel(PoolArgs a, const int64_t* __restrict__ idx) {
+  pdl_wait();
   // a.x = gy, a.y = gx; the windows that can hold input (y, xx): output rows ceil((y + p - KS + 1) / ST) .. floor((y + p) / ST)
   constexpr int NW = (KS + ST - 1) / ST;  // at most this many windows per axis
   const int c4 = a.c >> 2;
@@ -308,6 +318,7 @@ __global__ void __launch_bounds__(256) maxpool_bwd_nhwc4_fixed_kernel(PoolArgs a
 // (this kernel is bound by the bytes that cross L1, not by HBM). Indices are compared in 32 bits (h * w < 2^31).
 template <int KS>
 __global__ void __launch_bounds__(256) maxpool_bwd_nhwc4_s2_block_kernel(PoolArgs a, const int64_t* __restrict__ idx) {
+  pdl_wait();
   const int c4 = a.c >> 2, hb = (a.ih + 1) >> 1, wb = (a.iw + 1) >> 1;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)a.n * hb * wb * c4) return;
@@ -373,6 +384,7 @@ __device__ __forceinline__ float avg_div(const PoolArgs& a, int oy, int ox) {
 }
 template <bool NHWC>
 __global__ void __launch_bounds__(256) avgpool_fwd_kernel(PoolArgs a) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)a.n * a.c * a.oh * a.ow) return;
   int img, ch, oy, ox;
@@ -392,6 +404,7 @@ __global__ void __launch_bounds__(256) avgpool_fwd_kernel(PoolArgs a) {
 }
 template <bool NHWC>
 __global__ void __launch_bounds__(256) avgpool_bwd_kernel(PoolArgs a) {  // a.x = gy, a.y = gx
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)a.n * a.c * a.ih * a.iw) return;
   int img, ch, y, xx;
@@ -409,6 +422,7 @@ __device__ __forceinline__ int ad_start(int o, int I, int O) { return (int)(((in
 __device__ __forceinline__ int ad_end(int o, int I, int O) { return (int)((((int64_t)o + 1) * I + O - 1) / O); }
 template <bool NHWC>
 __global__ void __launch_bounds__(256) adapool_fwd_kernel(PoolArgs a) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)a.n * a.c * a.oh * a.ow) return;
   int img, ch, oy, ox;
@@ -422,6 +436,7 @@ __global__ void __launch_bounds__(256) adapool_fwd_kernel(PoolArgs a) {
 }
 // global average pool over an NCHW plane: one warp per (n, c) plane, coalesced, shuffle-reduced
 __global__ void __launch_bounds__(256) gap_nchw_kernel(const float* __restrict__ x, float* __restrict__ y, int64_t planes, int hw) {
+  pdl_wait();
   int64_t pl = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int lane = threadIdx.x & 31;
   if (pl >= planes) return;
@@ -433,6 +448,7 @@ __global__ void __launch_bounds__(256) gap_nchw_kernel(const float* __restrict__
 }
 template <bool NHWC>
 __global__ void __launch_bounds__(256) adapool_bwd_kernel(PoolArgs a) {  // a.x = gy, a.y = gx
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)a.n * a.c * a.ih * a.iw) return;
   int img, ch, y, xx;
@@ -466,8 +482,8 @@ static inline bool aligned16(const void* a, const void* b, const void* c) {
 #define LAUNCH_BY_LAYOUT(kern, nhwc, total, s, ...)                                      \
   do {                                                                                   \
     unsigned blocks_ = (unsigned)cdiv((total), 256);                                     \
-    if (nhwc) kern<true><<<blocks_, 256, 0, (s)>>>(__VA_ARGS__);                          \
-    else kern<false><<<blocks_, 256, 0, (s)>>>(__VA_ARGS__);                              \
+    if (nhwc) launch(kern<true>, blocks_, 256, 0, (s), __VA_ARGS__);                          \
+    else launch(kern<false>, blocks_, 256, 0, (s), __VA_ARGS__);                              \
   } while (0)
 
 }  // namespace omt
@@ -519,16 +535,16 @@ int omt_maxpool_fwd(const OmtAct* x, const OmtAct* y, int64_t* idx, int32_t n, i
     const int64_t total = (int64_t)n * oh * ow * (c / 4);
     const bool square = p->kh == p->kw && p->sh == p->sw && p->dh == 1 && p->dw == 1;
     if (square && p->kh == 3 && p->sh == 2) {
-      maxpool_fwd_nhwc4_fixed_kernel<3, 2, 4><<<(unsigned)cdiv((int64_t)n * oh * cdiv(ow, 4) * (c / 4), 256), 256, 0, st(stream)>>>(
+      launch(maxpool_fwd_nhwc4_fixed_kernel<3, 2, 4>, (unsigned)cdiv((int64_t)n * oh * cdiv(ow, 4) * (c / 4), 256), 256, 0, st(stream),
           pa(x, y, n, c, ih, iw, oh, ow, p, 0, 0), idx);
       return check_launch("maxpool_fwd_nhwc4_k3s2");
     }
     if (square && p->kh == 2 && p->sh == 2) {
-      maxpool_fwd_nhwc4_fixed_kernel<2, 2, 4><<<(unsigned)cdiv((int64_t)n * oh * cdiv(ow, 4) * (c / 4), 256), 256, 0, st(stream)>>>(
+      launch(maxpool_fwd_nhwc4_fixed_kernel<2, 2, 4>, (unsigned)cdiv((int64_t)n * oh * cdiv(ow, 4) * (c / 4), 256), 256, 0, st(stream),
           pa(x, y, n, c, ih, iw, oh, ow, p, 0, 0), idx);
       return check_launch("maxpool_fwd_nhwc4_k2s2");
     }
-    maxpool_fwd_nhwc4_kernel<<<(unsigned)cdiv(total, 256), 256, 0, st(stream)>>>(pa(x, y, n, c, ih, iw, oh, ow, p, 0, 0), idx);
+    launch(maxpool_fwd_nhwc4_kernel, (unsigned)cdiv(total, 256), 256, 0, st(stream), pa(x, y, n, c, ih, iw, oh, ow, p, 0, 0), idx);
     return check_launch("maxpool_fwd_nhwc4");
   }
   LAUNCH_BY_LAYOUT(maxpool_fwd_kernel, chan_last(y), (int64_t)n * c * oh * ow, st(stream), pa(x, y, n, c, ih, iw, oh, ow, p, 0, 0), idx);
@@ -544,14 +560,14 @@ int omt_maxpool_bwd(const OmtAct* gy, const int64_t* idx, const OmtAct* gx, int3
     const bool square = p->kh == p->kw && p->sh == p->sw && p->dh == 1 && p->dw == 1;
     const int64_t blocks2 = (int64_t)n * ((ih + 1) / 2) * ((iw + 1) / 2) * (c / 4);  // 2 x 2 pixel blocks x channel quads
     if (square && p->kh == 3 && p->sh == 2 && iw > 1) {
-      maxpool_bwd_nhwc4_s2_block_kernel<3><<<(unsigned)cdiv(blocks2, 256), 256, 0, st(stream)>>>(pa(gy, gx, n, c, ih, iw, oh, ow, p, 0, 0), idx);
+      launch(maxpool_bwd_nhwc4_s2_block_kernel<3>, (unsigned)cdiv(blocks2, 256), 256, 0, st(stream), pa(gy, gx, n, c, ih, iw, oh, ow, p, 0, 0), idx);
       return check_launch("maxpool_bwd_nhwc4_k3s2");
     }
     if (square && p->kh == 2 && p->sh == 2 && iw > 1) {
-      maxpool_bwd_nhwc4_s2_block_kernel<2><<<(unsigned)cdiv(blocks2, 256), 256, 0, st(stream)>>>(pa(gy, gx, n, c, ih, iw, oh, ow, p, 0, 0), idx);
+      launch(maxpool_bwd_nhwc4_s2_block_kernel<2>, (unsigned)cdiv(blocks2, 256), 256, 0, st(stream), pa(gy, gx, n, c, ih, iw, oh, ow, p, 0, 0), idx);
       return check_launch("maxpool_bwd_nhwc4_k2s2");
     }
-    maxpool_bwd_nhwc4_kernel<<<(unsigned)cdiv(total, 256), 256, 0, st(stream)>>>(pa(gy, gx, n, c, ih, iw, oh, ow, p, 0, 0), idx);
+    launch(maxpool_bwd_nhwc4_kernel, (unsigned)cdiv(total, 256), 256, 0, st(stream), pa(gy, gx, n, c, ih, iw, oh, ow, p, 0, 0), idx);
     return check_launch("maxpool_bwd_nhwc4");
   }
   LAUNCH_BY_LAYOUT(maxpool_bwd_kernel, chan_last(gx), (int64_t)n * c * ih * iw, st(stream), pa(gy, gx, n, c, ih, iw, oh, ow, p, 0, 0),
@@ -581,7 +597,7 @@ int omt_adaptive_avgpool_fwd(const OmtAct* x, const OmtAct* y, int32_t n, int32_
   OMT_REQUIRE(x && y && x->p && y->p && n > 0 && c > 0 && ih > 0 && iw > 0 && oh > 0 && ow > 0, "omt_adaptive_avgpool_fwd: bad arguments");
   if (oh == 1 && ow == 1 && is_nchw(x, c, ih, iw) && y->sc == 1 && y->sn == c) {
     int64_t planes = (int64_t)n * c;
-    gap_nchw_kernel<<<(unsigned)cdiv(planes * 32, 256), 256, 0, st(stream)>>>(x->p, y->p, planes, ih * iw);
+    launch(gap_nchw_kernel, (unsigned)cdiv(planes * 32, 256), 256, 0, st(stream), x->p, y->p, planes, ih * iw);
     return check_launch("gap_fwd_nchw");
   }
   LAUNCH_BY_LAYOUT(adapool_fwd_kernel, chan_last(y) || (oh == 1 && ow == 1 && chan_last(x)), (int64_t)n * c * oh * ow, st(stream),

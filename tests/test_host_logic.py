@@ -318,3 +318,26 @@ def test_conv_plan_overrides_round_trip_without_a_gpu():
         f = [int(v) for v in k.split(",")]
         capi.call("omt_conv_plan_set", f[0], capi.geo(f[1], f[2], f[3], f[4], f[5], f[8], f[9], f[10]), 0, 1.0)
     assert capi.conv_plans_dump() == {}
+
+
+def test_every_kernel_waits_for_the_kernel_in_front():
+    """Kernels are launched with programmatic stream serialisation, which is only ordinary stream order while each of them
+    executes pdl_wait() before anything else that touches global memory (the two tensor-core kernels: after their setup of
+    barriers and tensor memory) and no launch goes around launch()."""
+    import pathlib
+    import re
+    for src in sorted((pathlib.Path(__file__).resolve().parents[1] / "omarchy_mac_torch_b200" / "csrc").glob("*.cu")):
+        text = src.read_text()
+        assert "<<<" not in text, src.name
+        for m in re.finditer(r"__global__", text):
+            decl = text[m.start():text.index("{", m.start())]
+            if ";" in decl:
+                continue  # a declaration
+            body = re.sub(r"//[^\n]*", "", text[m.start() + len(decl) + 1:]).lstrip()
+            name = re.search(r"(\w+)\(", re.sub(r"__launch_bounds__\([^)]*\)", "", decl)).group(1)
+            if name in ("conv_tc_kernel", "wgrad_tc_kernel"):
+                head = body[:body.index("pdl_wait();")]
+                assert not any(w in head for w in ("cp_async", "tma_", "__ldg", "g.y.", "g.part", "g.stats", "g.bias")), name
+            else:
+                assert body.startswith("pdl_wait();"), name
+        assert len(re.findall(r"cudaLaunchKernelEx\(", text)) == text.count(", pdl_attr()}"), src.name
