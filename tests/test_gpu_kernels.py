@@ -859,3 +859,17 @@ def test_bn_fold_equals_the_elementwise_ops(capi, co, ci, ks, bias):
     scale = gamma * torch.rsqrt(rv + 1e-5)
     assert torch.equal(fw, w * scale.view(-1, 1, 1, 1))
     assert torch.equal(fb, ((cb - rm) if bias else -rm) * scale + beta)
+
+
+@pytest.mark.parametrize("n,c,h,w", [(1, 2, 1, 1), (3, 5, 7, 9), (32, 24, 1, 1), (2, 66, 31, 17), (16, 64, 55, 55), (1, 260, 40, 40), (2, 1024, 9, 7), (7, 130, 63, 50)])
+def test_bias_gradient_of_channels_last_tensors(capi, n, c, h, w):
+    """One and several slices, 16-byte and single-float lanes, one to several channel blocks, pixel counts that divide nothing.
+    A sum of k terms in float32 is within k * 2^-24 of sum |x|; the lanes add at most k / 256 terms one after the other."""
+    gy = torch.randn(n, c, h, w, generator=torch.Generator().manual_seed(c)).contiguous(memory_format=torch.channels_last).cuda()
+    ref = gy.double().sum((0, 2, 3))
+    bound = gy.double().abs().sum((0, 2, 3)) * (n * h * w / 256 + 64) * 2.0**-24
+    for scale in (1.0, -0.5):
+        assert ((capi.conv_bias_grad(gy, scale).double() - scale * ref).abs() <= bound * abs(scale)).all()
+    off = torch.zeros(gy.numel() + 1, device="cuda")[1:].view(n, h, w, c).permute(0, 3, 1, 2)  # 4 bytes past a 16-byte boundary
+    off.copy_(gy)
+    assert ((capi.conv_bias_grad(off).double() - ref).abs() <= bound).all()
