@@ -7,6 +7,7 @@
 // of the K loop (rows/columns are decomposed once per thread, the K index once per thread per step), register
 // prefetch with double-buffered shared tiles, 128-bit shared loads and stores.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -28,7 +29,7 @@ constexpr int BK = 8;
 
 // ---- forward: m=(img,oy,ox) k=(ci,ky,kx) n=co ---------------------------------------------------------------------
 struct Fwd {
-  static constexpr bool A_MFAST = true, B_NFAST = false;
+  static constexpr bool A_MFAST = true, B_NFAST = false, SEQ = false;
   const ConvArgs& g;
   int M, N, kbeg, kend;
   __device__ Fwd(const ConvArgs& g_, int) : g(g_), M(g_.M), N(g_.N), kbeg(0), kend(g_.K) {}
@@ -108,7 +109,7 @@ struct Fwd {
 // Phase (py,px) covers input pixels y=py+s*i, x=px+s*j. Only taps ky=ky0+s*ty, kx=kx0+s*tx reach them, from output
 // pixel (i+qy-ty, j+qx-tx). Same index algebra as the reference host loop (csrc/conv.cpp:78-95).
 struct Dgrad {
-  static constexpr bool A_MFAST = true, B_NFAST = true;
+  static constexpr bool A_MFAST = true, B_NFAST = true, SEQ = false;
   const ConvArgs& g;
   int M, N, kbeg, kend;
   int py, px, ky0, kx0, qy, qx, hi, wi, jy, jx;
@@ -175,7 +176,7 @@ struct Dgrad {
 
 // ---- weight gradient, one K slice per blockIdx.z: m=co k=(img,oy,ox) n=(ci,ky,kx) -------------------------------------
 struct Wgrad {
-  static constexpr bool A_MFAST = false, B_NFAST = false;
+  static constexpr bool A_MFAST = false, B_NFAST = false, SEQ = false;
   const ConvArgs& g;
   int M, N, kbeg, kend, z;
   __device__ Wgrad(const ConvArgs& g_, int z_) : g(g_), M(g_.M), N(g_.N), z(z_) {
@@ -216,29 +217,150 @@ struct Wgrad {
   }
 };
 
-// C tile BM x BN per block of 256 threads; each thread owns TM x TN as (TM/4) x (TN/4) groups of 4x4, groups BM/2 or
-// BN/2 apart, threads m-fastest so stores along m coalesce for NCHW outputs.
-template <class L, int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__(256) conv_gemm_simt(ConvArgs g) {
+// ---- channels-last operands ---------------------------------------------------------------------------------------------
+// The loaders above walk the reduction as (channel, ky, kx): neighbouring lanes then read a channel count apart in a channels-last
+// tensor, one sector per float. These walk it as (block of 8 channels, ky, kx, channel), 8 lanes to a pixel's channels, so that a
+// sector is used whole; the taps of one channel block follow each other, so that their weights (ks * ks consecutive floats per
+// channel) and the shifted rows of the activation are still in L1. A thread's position advances tap by tap: no division per step.
+struct FwdCl : Fwd {
+  static constexpr bool A_MFAST = false, B_NFAST = false, SEQ = true;
+  __device__ FwdCl(const ConvArgs& g_, int z) : Fwd(g_, z) { kend = (g_.ci + 7) / 8 * 8 * g_.ks * g_.ks; }
+  struct KIdx { int64_t off; int ky, kx, c, wofs; };
+  __device__ KIdx kidx(int k) const {  // k: any multiple of 8 plus the lane's channel
+    const int kk = g.ks * g.ks, step = k >> 3, blk = step / kk, tap = step - blk * kk, ky = tap / g.ks, kx = tap - ky * g.ks, c = blk * 8 + (k & 7);
+    return {c * g.a.sc + ky * g.a.sh + kx * g.a.sw, ky, kx, c, c * kk + tap};
+  }
+  __device__ void advance(KIdx& k) const {
+    k.kx++; k.wofs++; k.off += g.a.sw;
+    if (k.kx == g.ks) {
+      k.kx = 0; k.ky++; k.off += g.a.sh - g.ks * g.a.sw;
+      if (k.ky == g.ks) { k.ky = 0; k.c += 8; k.off += 8 * g.a.sc - g.ks * g.a.sh; k.wofs += 7 * g.ks * g.ks; }
+    }
+  }
+  __device__ float loadA(const Row& r, const KIdx& k) const {
+    const int y = r.iy0 + k.ky, x = r.ix0 + k.kx;
+    return k.c < g.ci && (unsigned)y < (unsigned)g.ih && (unsigned)x < (unsigned)g.iw ? __ldg(g.a.p + r.base + k.off) : 0.f;
+  }
+  __device__ float loadB(const Col& c, const KIdx& k, int) const { return c.p && k.c < g.ci ? __ldg(c.p + k.wofs) : 0.f; }
+  __device__ void store(int m, int nn, const float (&v)[4][4]) const {
+    const int ohw = g.oh * g.ow;
+    float bv[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) bv[j] = (g.flags & OMT_EPI_BIAS) && nn + j < N ? __ldg(g.bias + nn + j) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      if (m + i >= M) break;
+      const int img = (m + i) / ohw, r = m + i - img * ohw, oy = r / g.ow, ox = r - oy * g.ow;
+      float* p = g.b.p + g.b.off(img, nn, oy, ox);
+      float o[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        o[j] = v[i][j] + bv[j];
+        if (g.flags & OMT_EPI_RELU) o[j] = fmaxf(o[j], 0.f);
+      }
+      if (nn + 3 < N && (reinterpret_cast<uintptr_t>(p) & 15) == 0) *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]);
+      else {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          if (nn + j < N) p[j] = o[j];
+      }
+    }
+  }
+};
+
+struct DgradCl : Dgrad {
+  static constexpr bool A_MFAST = false, B_NFAST = true, SEQ = true;
+  __device__ DgradCl(const ConvArgs& g_, int z) : Dgrad(g_, z) { kend = (g_.co + 7) / 8 * 8 * jy * jx; }
+  struct KIdx { int64_t off; int ty, tx, c, wofs; };
+  __device__ int wofs_of(int c, int ty, int tx) const { return (c * g.ci * g.ks + ky0 + g.stride * ty) * g.ks + kx0 + g.stride * tx; }
+  __device__ KIdx kidx(int k) const {
+    const int jj = max(1, jy * jx), step = k >> 3, blk = step / jj, tap = step - blk * jj, ty = tap / max(1, jx), tx = tap - ty * jx, c = blk * 8 + (k & 7);
+    return {c * g.a.sc - ty * g.a.sh - tx * g.a.sw, ty, tx, c, wofs_of(c, ty, tx)};
+  }
+  __device__ void advance(KIdx& k) const {
+    k.tx++; k.off -= g.a.sw;
+    if (k.tx == jx) {
+      k.tx = 0; k.ty++; k.off += jx * g.a.sw - g.a.sh;
+      if (k.ty == jy) { k.ty = 0; k.c += 8; k.off += 8 * g.a.sc + jy * g.a.sh; }
+    }
+    k.wofs = wofs_of(k.c, k.ty, k.tx);
+  }
+  __device__ float loadA(const Row& r, const KIdx& k) const {
+    const int oy = r.oy0 - k.ty, ox = r.ox0 - k.tx;
+    return k.c < g.co && (unsigned)oy < (unsigned)g.oh && (unsigned)ox < (unsigned)g.ow ? __ldg(g.a.p + r.base + k.off) : 0.f;
+  }
+  __device__ float loadB(const Col& c, const KIdx& k, int) const { return c.ok && k.c < g.co ? __ldg(g.w + k.wofs + c.wofs) : 0.f; }
+  __device__ void store(int m, int nn, const float (&v)[4][4]) const {  // (neighbouring threads hold neighbouring columns: see the kernel)
+    const int hw = hi * wi;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      if (m + i >= M) break;
+      const int img = (m + i) / hw, r = m + i - img * hw, ii = r / wi, jj = r - ii * wi;
+      float* p = g.b.p + g.b.off(img, nn, py + g.stride * ii, px + g.stride * jj);
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (nn + j < N) p[j] = v[i][j];
+    }
+  }
+};
+
+// columns as (tap, channel): neighbouring lanes read neighbouring channels of x; the stores put them back into [ci][ky][kx]
+struct WgradCl : Wgrad {
+  static constexpr bool A_MFAST = true, B_NFAST = true, SEQ = false;
+  using Wgrad::Wgrad;
+  __device__ Col col(int nn) const {
+    if (nn >= N) return {0, 0, 0, false};
+    const int tap = nn / g.ci, c = nn - tap * g.ci, ky = tap / g.ks, kx = tap - ky * g.ks;
+    return {c * g.b.sc + ky * g.b.sh + kx * g.b.sw, ky, kx, true};
+  }
+  __device__ void store(int m, int nn, const float (&v)[4][4]) const {
+    float* base = g.out + (int64_t)z * M * N;
+    const float sc = g.slices == 1 ? g.scale : 1.f;
+    const int kk = g.ks * g.ks;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      if (nn + j >= N) break;
+      const int tap = (nn + j) / g.ci, c = nn + j - tap * g.ci;
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (m + i < M) base[(int64_t)(m + i) * N + c * kk + tap] = v[i][j] * sc;
+    }
+  }
+};
+
+// C tile BM x BN, KG groups of (BM / TM) * (BN / TN) threads. Each thread of a group owns TM x TN outputs as (TM/4) x (TN/4) groups of
+// 4x4, groups BM/2 or BN/2 apart, threads m-fastest so stores along m coalesce for NCHW outputs. The KG groups work on the
+// same tile and take every KG-th step of the reduction, each with its own shared tiles; their sums meet in shared memory, in group
+// order, at the end. That is for launches with fewer tiles than the SMs need warps (KG = 2) and for weight gradients of a few
+// outputs over very many pixels (16 x 32 outputs, eight groups), which a 128 x 64 tile computes almost entirely as padding: 252 us
+// for 16 x 27 outputs over 401 408 pixels, 7 % of a MobileNetV3 step. With the channels-last loaders the three passes of a
+// 90 -> 50 channel 3x3 stride-2 layer (13 x 57 x 43) go from 217 to 151 us, that step from 3783 to 3592.
+template <class L, int BM, int BN, int TM, int TN, int KG = 1>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN) * KG, L::SEQ && BM * BN == 128 * 128 ? 2 : 1) conv_gemm_simt(ConvArgs g) {
   pdl_wait();
-  constexpr int TY = BM / TM, GM = TM / 4, GN = TN / 4;
-  constexpr int RA = BM / 32, RB = (BN + 31) / 32;
-  static_assert((BM / TM) * (BN / TN) == 256, "256 threads");
-  __shared__ __align__(16) float As[2][BK][BM + 4];
-  __shared__ __align__(16) float Bs[2][BK][BN + 4];
+  constexpr int TY = BM / TM, GM = TM / 4, GN = TN / 4, TG = (BM / TM) * (BN / TN);
+  constexpr bool A_MF = L::A_MFAST && TG == 256, B_NF = L::B_NFAST && TG == 256;  // small groups: lanes along k, one position per thread
+  constexpr int RS = TG / 8;  // rows (columns) that one pass of a group's threads covers
+  constexpr int RA = BM / RS, RB = (BN + RS - 1) / RS;
+  static_assert(BM % RS == 0 && (TG == 256 || BN % RS == 0), "whole passes");
+  constexpr int TILE_F = 2 * BK * (BM + 4) + 2 * BK * (BN + 4);
+  constexpr int SMEM_F = KG > 1 && BM * BN > KG * TILE_F ? BM * BN : KG * TILE_F;
+  __shared__ __align__(16) float sm[SMEM_F];
+  const int kg = KG > 1 ? threadIdx.x / TG : 0, tid = KG > 1 ? threadIdx.x % TG : threadIdx.x;
+  float (*As)[BK][BM + 4] = reinterpret_cast<float (*)[BK][BM + 4]>(sm + kg * TILE_F);
+  float (*Bs)[BK][BN + 4] = reinterpret_cast<float (*)[BK][BN + 4]>(sm + kg * TILE_F + 2 * BK * (BM + 4));
   L ld(g, blockIdx.z);
   const int M = ld.M, N = ld.N;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;  // M tiles on x: its limit is 2^31-1, y's is 65535
   if (m0 >= M) return;
-  const int tid = threadIdx.x;
-  const int a_k = L::A_MFAST ? (tid >> 5) : (tid & 7), a_r = L::A_MFAST ? (tid & 31) : (tid >> 3);
-  const int b_k = L::B_NFAST ? (tid >> 5) : (tid & 7), b_r = L::B_NFAST ? (tid & 31) : (tid >> 3);
+  const int a_k = A_MF ? (tid >> 5) : (tid & 7), a_r = A_MF ? (tid & 31) : (tid >> 3);
+  const int b_k = B_NF ? (tid >> 5) : (tid & 7), b_r = B_NF ? (tid & 31) : (tid >> 3);
   typename L::Row ra[RA];
   typename L::Col cb[RB];
 #pragma unroll
-  for (int i = 0; i < RA; i++) ra[i] = ld.row(m0 + a_r + 32 * i);
+  for (int i = 0; i < RA; i++) ra[i] = ld.row(m0 + a_r + RS * i);
 #pragma unroll
-  for (int i = 0; i < RB; i++) cb[i] = ld.col((b_r + 32 * i < BN) ? n0 + b_r + 32 * i : N);
+  for (int i = 0; i < RB; i++) cb[i] = ld.col((b_r + RS * i < BN) ? n0 + b_r + RS * i : N);
   float acc[GM][GN][4][4];
 #pragma unroll
   for (int a = 0; a < GM; a++)
@@ -249,36 +371,46 @@ __global__ void __launch_bounds__(256) conv_gemm_simt(ConvArgs g) {
 #pragma unroll
         for (int j = 0; j < 4; j++) acc[a][b][i][j] = 0.f;
   float pa[RA], pb[RB];
+  typename L::KIdx ka = ld.kidx(ld.kbeg + kg * BK + a_k), kb = ld.kidx(ld.kbeg + kg * BK + b_k);  // (SEQ loaders: the position to fetch next)
   auto fetch = [&](int k0) {
-    typename L::KIdx ka = ld.kidx(k0 + a_k);
+    if constexpr (!L::SEQ) {
+      ka = ld.kidx(k0 + a_k);
+      if constexpr (A_MF != B_NF) kb = ld.kidx(k0 + b_k);
+    }
 #pragma unroll
     for (int i = 0; i < RA; i++) pa[i] = ld.loadA(ra[i], ka);
-    if constexpr (L::A_MFAST == L::B_NFAST) {
+    if constexpr (A_MF == B_NF) {
 #pragma unroll
       for (int i = 0; i < RB; i++) pb[i] = ld.loadB(cb[i], ka, k0 + b_k);
     } else {
-      typename L::KIdx kb = ld.kidx(k0 + b_k);
 #pragma unroll
       for (int i = 0; i < RB; i++) pb[i] = ld.loadB(cb[i], kb, k0 + b_k);
+    }
+    if constexpr (L::SEQ) {
+#pragma unroll
+      for (int q = 0; q < KG; q++) {
+        ld.advance(ka);
+        if constexpr (A_MF != B_NF) ld.advance(kb);
+      }
     }
   };
   auto commit = [&](int buf) {
 #pragma unroll
-    for (int i = 0; i < RA; i++) As[buf][a_k][a_r + 32 * i] = pa[i];
+    for (int i = 0; i < RA; i++) As[buf][a_k][a_r + RS * i] = pa[i];
 #pragma unroll
     for (int i = 0; i < RB; i++)
-      if (b_r + 32 * i < BN) Bs[buf][b_k][b_r + 32 * i] = pb[i];
+      if (b_r + RS * i < BN) Bs[buf][b_k][b_r + RS * i] = pb[i];
   };
   const int tm = tid % TY, tn = tid / TY;
   int buf = 0;
-  if (ld.kbeg < ld.kend) {
-    fetch(ld.kbeg);
+  if (ld.kbeg < ld.kend) {  // (loads at and beyond kend give zeros: the last round of the groups may be partly empty)
+    fetch(ld.kbeg + kg * BK);
     commit(0);
   }
   __syncthreads();
-  for (int k0 = ld.kbeg; k0 < ld.kend; k0 += BK) {
-    const bool more = k0 + BK < ld.kend;
-    if (more) fetch(k0 + BK);
+  for (int k0 = ld.kbeg; k0 < ld.kend; k0 += BK * KG) {
+    const bool more = k0 + BK * KG < ld.kend;
+    if (more) fetch(k0 + BK * KG + kg * BK);
 #pragma unroll
     for (int kk = 0; kk < BK; kk++) {
       float4 av[GM], bv[GN];
@@ -303,6 +435,26 @@ __global__ void __launch_bounds__(256) conv_gemm_simt(ConvArgs g) {
     __syncthreads();
     buf ^= 1;
   }
+  if constexpr (KG > 1) {
+    static_assert(GM == 1 && GN == 1, "one 4x4 group per thread");
+    float4* red = reinterpret_cast<float4*>(sm);  // [4][TG] float4: one group's tile at a time
+    for (int q = 1; q < KG; q++) {
+      if (kg == q) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) red[i * TG + tid] = make_float4(acc[0][0][i][0], acc[0][0][i][1], acc[0][0][i][2], acc[0][0][i][3]);
+      }
+      __syncthreads();
+      if (kg == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const float4 v = red[i * TG + tid];
+          acc[0][0][i][0] += v.x; acc[0][0][i][1] += v.y; acc[0][0][i][2] += v.z; acc[0][0][i][3] += v.w;
+        }
+      }
+      __syncthreads();
+    }
+    if (kg != 0) return;
+  }
 #pragma unroll
   for (int a = 0; a < GM; a++)
 #pragma unroll
@@ -323,27 +475,38 @@ __global__ void __launch_bounds__(256) slab_sum_kernel(const float* __restrict__
   out[i] = s * scale;
 }
 
+template <class L, int BM, int BN, int TM, int TN, int KG = 1>
+static void launch_tile(const ConvArgs& a, int64_t Mmax, int64_t N, int gz, cudaStream_t s) {
+  const dim3 grid((unsigned)cdiv(Mmax, BM), (unsigned)cdiv(N, BN), gz);
+  launch(conv_gemm_simt<L, BM, BN, TM, TN, KG>, grid, (BM / TM) * (BN / TN) * KG, 0, s, a);
+}
 template <class L>
 static int launch_gemm(const ConvArgs& a, int64_t Mmax, int64_t N, int gz, cudaStream_t s, const char* name) {
+  constexpr bool WGRAD = std::is_base_of_v<Wgrad, L>;
   // tile choice: narrow-N tiles for tiny channel counts, smaller tiles when the grid would not fill the SMs
   int sms = sm_count();
   auto blocks = [&](int bm, int bn) { return cdiv(Mmax, bm) * cdiv(N, bn) * gz; };
   // M tiles on grid.x (limit 2^31-1), N tiles on grid.y (limit 65535: N is a channel count, or ci*ks*ks for the weight gradient)
   OMT_REQUIRE(cdiv(N, N <= 16 ? 16 : 64) <= 65535 && gz <= 65535, "%s: %lld GEMM columns exceed the launch grid", name, (long long)N);
+  if constexpr (WGRAD) {
+    bool done = true;
+    if (Mmax <= 16 && N <= 32) launch_tile<L, 16, 32, 4, 4, 8>(a, Mmax, N, gz, s);  // a few outputs (first layers): small tiles, the reduction
+    else if (Mmax <= 32 && N <= 32) launch_tile<L, 32, 32, 4, 4, 4>(a, Mmax, N, gz, s);  // shared by the block's groups
+    else if (Mmax <= 64 && N > 64 && blocks(128, 128) >= sms) launch_tile<L, 64, 128, 4, 8>(a, Mmax, N, gz, s);
+    else done = false;
+    if (done) return check_launch(name);
+  }
   if (N <= 16) {
-    dim3 grid((unsigned)cdiv(Mmax, 256), (unsigned)cdiv(N, 16), gz);
-    launch(conv_gemm_simt<L, 256, 16, 4, 4>, grid, 256, 0, s, a);
+    launch_tile<L, 256, 16, 4, 4>(a, Mmax, N, gz, s);
   } else if (N <= 64 || blocks(128, 128) < sms) {
     if (blocks(128, 64) < sms) {
-      dim3 grid((unsigned)cdiv(Mmax, 64), (unsigned)cdiv(N, 64), gz);
-      launch(conv_gemm_simt<L, 64, 64, 4, 4>, grid, 256, 0, s, a);
+      if (blocks(64, 64) <= sms) launch_tile<L, 64, 64, 4, 4, 2>(a, Mmax, N, gz, s);  // one block per SM at most: twice the warps
+      else launch_tile<L, 64, 64, 4, 4>(a, Mmax, N, gz, s);
     } else {
-      dim3 grid((unsigned)cdiv(Mmax, 128), (unsigned)cdiv(N, 64), gz);
-      launch(conv_gemm_simt<L, 128, 64, 8, 4>, grid, 256, 0, s, a);
+      launch_tile<L, 128, 64, 8, 4>(a, Mmax, N, gz, s);
     }
   } else {
-    dim3 grid((unsigned)cdiv(Mmax, 128), (unsigned)cdiv(N, 128), gz);
-    launch(conv_gemm_simt<L, 128, 128, 8, 8>, grid, 256, 0, s, a);
+    launch_tile<L, 128, 128, 8, 8>(a, Mmax, N, gz, s);
   }
   return check_launch(name);
 }
@@ -361,6 +524,8 @@ int simt_conv_fwd(const OmtConvGeo* g, const OmtAct* x, const float* w, const fl
   ConvArgs a = base_args(g);
   a.a = view(x); a.b = view(y); a.w = w; a.bias = bias; a.flags = flags;
   a.M = g->n * g->oh * g->ow; a.N = g->co; a.K = g->ci * g->ks * g->ks;
+  // (channels-last on both sides; below 8 input channels a step of 8 would mostly be padding)
+  if (x->sc == 1 && y->sc == 1 && g->ci >= 8) return launch_gemm<FwdCl>(a, a.M, a.N, 1, s, "conv_fwd_simt");
   return launch_gemm<Fwd>(a, a.M, a.N, 1, s, "conv_fwd_simt");
 }
 
@@ -464,6 +629,7 @@ int simt_conv_dgrad(const OmtConvGeo* g, const OmtAct* gy, const float* w, const
   int st_ = g->stride;
   int64_t hi = cdiv(g->ih, st_), wi = cdiv(g->iw, st_);  // phase (0,0) is the largest
   a.N = g->ci;
+  if (gy->sc == 1 && dx->sc == 1 && g->co >= 8) return launch_gemm<DgradCl>(a, (int64_t)g->n * hi * wi, a.N, st_ * st_, s, "conv_dgrad_simt");
   return launch_gemm<Dgrad>(a, (int64_t)g->n * hi * wi, a.N, st_ * st_, s, "conv_dgrad_simt");
 }
 
@@ -488,7 +654,8 @@ int simt_conv_wgrad(const OmtConvGeo* g, const OmtAct* x, const OmtAct* gy, floa
   a.M = g->co; a.N = g->ci * g->ks * g->ks; a.K = g->n * g->oh * g->ow;
   wgrad_slices(g, &a.slices, &a.kslice);
   a.out = a.slices == 1 ? dw : part;
-  int r = launch_gemm<Wgrad>(a, a.M, a.N, a.slices, s, "conv_wgrad_simt");
+  int r = x->sc == 1 && gy->sc == 1 && g->ci >= 8 ? launch_gemm<WgradCl>(a, a.M, a.N, a.slices, s, "conv_wgrad_simt")
+                                                  : launch_gemm<Wgrad>(a, a.M, a.N, a.slices, s, "conv_wgrad_simt");
   if (r != OMT_OK || a.slices == 1) return r;
   int64_t total = (int64_t)a.M * a.N;
   launch(slab_sum_kernel, (unsigned)cdiv(total, 256), 256, 0, s, part, dw, total, a.slices, scale);

@@ -873,3 +873,34 @@ def test_bias_gradient_of_channels_last_tensors(capi, n, c, h, w):
     off = torch.zeros(gy.numel() + 1, device="cuda")[1:].view(n, h, w, c).permute(0, 3, 1, 2)  # 4 bytes past a 16-byte boundary
     off.copy_(gy)
     assert ((capi.conv_bias_grad(off).double() - ref).abs() <= bound).all()
+
+
+SIMT_CL = [  # n, ci, co, h, w, ks, stride, pad: channel counts around the step of 8, tiles of 64 and 128 in rows and columns, ragged sizes, empty stride phases
+    (1, 9, 9, 5, 5, 3, 1, 1), (2, 15, 17, 7, 9, 1, 1, 0), (13, 90, 50, 57, 43, 3, 2, 1), (3, 41, 130, 20, 19, 3, 1, 1), (2, 10, 9, 12, 8, 1, 3, 0), (5, 66, 70, 40, 33, 5, 1, 2),
+    (2, 9, 65, 9, 9, 7, 4, 5), (1, 257, 33, 6, 6, 3, 1, 1), (16, 130, 129, 30, 30, 1, 2, 0), (2, 5, 14, 16, 16, 3, 1, 1), (6, 3, 16, 40, 40, 3, 2, 1), (4, 1, 16, 28, 28, 3, 1, 1), (4, 3, 30, 31, 29, 3, 1, 1),
+]
+
+
+@pytest.mark.parametrize("cl", [False, True], ids=["nchw", "nhwc"])
+@pytest.mark.parametrize("case", SIMT_CL, ids=lambda t: "x".join(map(str, t)))
+def test_exact_float32_convolutions_vs_aten(capi, case, cl):
+    """The CUDA-core kernels in both layouts against float64 aten, bounded by (k + 2) 2^-24 of the sum of the absolute products
+    (k: the length of the reduction)."""
+    n, ci, co, h, w, ks, s, p = case
+    gen = torch.Generator().manual_seed(sum(case))
+    x, wt, b = torch.randn(n, ci, h, w, generator=gen), torch.randn(co, ci, ks, ks, generator=gen), torch.randn(co, generator=gen)
+    xd, wd = x.double().requires_grad_(), wt.double().requires_grad_()
+    y = torch.nn.functional.conv2d(xd, wd, b.double(), s, p)
+    gy = torch.randn(y.shape, generator=gen)
+    dx, dw = torch.autograd.grad(y, [xd, wd], gy.double())
+    xa, wa = x.double().abs().requires_grad_(), wt.double().abs().requires_grad_()
+    ya = torch.nn.functional.conv2d(xa, wa, b.double().abs(), s, p)
+    dxa, dwa = torch.autograd.grad(ya, [xa, wa], gy.double().abs())
+    eps = 2.0**-24
+    xc, gc = dev(x, cl), dev(gy, cl)
+    got = host(capi.conv_fwd(xc, wt.cuda(), b.cuda(), s, p, flags=capi.FORCE_SIMT | capi.EPI_RELU, cl=cl)).astype(np.float64)
+    assert (np.abs(got - y.detach().relu().numpy()) <= (ci * ks * ks + 2) * eps * ya.detach().numpy() + 1e-30).all()
+    got = host(capi.conv_dgrad(gc, wt.cuda(), (h, w), s, p, flags=capi.FORCE_SIMT, cl=cl)).astype(np.float64)
+    assert (np.abs(got - dx.numpy()) <= (co * ks * ks + 2) * eps * dxa.numpy() + 1e-30).all()
+    got = host(capi.conv_wgrad(xc, gc, ks, s, p, flags=capi.FORCE_SIMT, scale=0.5)).astype(np.float64)
+    assert (np.abs(got - 0.5 * dw.numpy()) <= (n * y.shape[2] * y.shape[3] + 2) * eps * 0.5 * dwa.numpy() + 1e-30).all()
