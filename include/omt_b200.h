@@ -347,6 +347,9 @@ int omt_sgd(const OmtParam* table, int32_t count, float lr, float momentum, floa
 /* Adam / AdamW (decoupled=1), adam.wgsl:13-27: bias corrections from the device step counter. */
 int omt_adam(const OmtParam* table, int32_t count, float lr, float beta1, float beta2, float eps,
              float weight_decay, int32_t decoupled, int32_t maximize, omt_stream_t stream);
+/* *ptrs[i] += value for `count` single floats on the device (the step counters that torch.optim advances in front of
+ * omt_adam; the reference adds them one dispatch each, csrc/optim.cpp). The entries must be distinct. */
+int omt_add_list(float* const* ptrs, int32_t count, float value, omt_stream_t stream);
 
 /* ---- fused pointwise chains: reference omt::fused_pointwise (csrc/fused.cpp:139-170) + compile pass 4 ---------------- */
 

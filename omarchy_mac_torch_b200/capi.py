@@ -121,6 +121,7 @@ SIGNATURES = {
     "omt_adaptive_avgpool_bwd": (_I, [_A, _A, _I, _I, _I, _I, _I, _I, _P]),
     "omt_sgd": (_I, [C.POINTER(Param), _I, _F, _F, _F, _F, _I, _I, _I, _P]),
     "omt_adam": (_I, [C.POINTER(Param), _I, _F, _F, _F, _F, _F, _I, _I, _P]),
+    "omt_add_list": (_I, [_P, _I, _F, _P]),
     "omt_scale_copy": (_I, [_P, _P, _I64, _F, _P]),
     "omt_act_copy": (_I, [_A, _A, _I, _I, _I, _I, _P]),
 }

@@ -56,6 +56,17 @@ static void fused_adamw_(at::TensorList params, at::TensorList grads, at::Tensor
 // kernel for this device that op decomposes into one add per tensor (one launch per parameter); here the whole list goes
 // through ATen's multi-tensor CUDA kernel on aliases of the same memory: one or two launches.
 static void foreach_add_scalar_(at::TensorList self, const at::Scalar& scalar) {
+  // Counters are single floats: one launch of the library's own, their addresses as its parameters, and no CUDA alias per tensor.
+  // (AdamW over 160 tensors, 64 M parameters, was bound by the host: 392 us a step, 281 with this and the kernel's 273.)
+  bool counters = !self.empty() && !scalar.isComplex();
+  for (const Tensor& t : self) counters = counters && f32(t) && t.numel() == 1;
+  if (counters) {
+    std::vector<float*> ptrs;
+    ptrs.reserve(self.size());
+    for (const Tensor& t : self) ptrs.push_back(t.data_ptr<float>());
+    check(omt_add_list(ptrs.data(), (int)ptrs.size(), scalar.to<float>(), cur_stream()), "step counters");
+    return;
+  }
   std::vector<Tensor> alias;
   alias.reserve(self.size());
   for (const Tensor& t : self) {

@@ -904,3 +904,15 @@ def test_exact_float32_convolutions_vs_aten(capi, case, cl):
     assert (np.abs(got - dx.numpy()) <= (co * ks * ks + 2) * eps * dxa.numpy() + 1e-30).all()
     got = host(capi.conv_wgrad(xc, gc, ks, s, p, flags=capi.FORCE_SIMT, scale=0.5)).astype(np.float64)
     assert (np.abs(got - 0.5 * dw.numpy()) <= (n * y.shape[2] * y.shape[3] + 2) * eps * 0.5 * dwa.numpy() + 1e-30).all()
+
+
+@pytest.mark.parametrize("count", [0, 1, 128, 439, 440, 441, 1000])
+def test_add_list(capi, count):
+    """One value added to each of a list of single floats, around the entries that one launch takes."""
+    import ctypes as C
+    t = torch.arange(2 * count + 1, dtype=torch.float32, device="cuda")
+    ptrs = (C.c_void_p * max(count, 1))(*[t.data_ptr() + 8 * i for i in range(count)])
+    capi.call("omt_add_list", ptrs, count, 2.5, capi.stream_handle())
+    want = torch.arange(2 * count + 1, dtype=torch.float32)
+    want[0:2 * count:2] += 2.5
+    assert torch.equal(t.cpu(), want)
