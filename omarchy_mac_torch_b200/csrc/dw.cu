@@ -9,17 +9,9 @@
 #include <mutex>
 #include <type_traits>
 
-#include "common.cuh"
+#include "dw.cuh"
 
 namespace omt {
-
-struct DwArgs {
-  ActView x, y;  // fwd: x in, y out. dgrad: x = gy (in), y = dx (out). wgrad: x = x, y = gy.
-  const float* w;
-  const float* bias;
-  int n, c, ih, iw, oh, ow, ks, stride, pad;
-  uint32_t flags;
-};
 
 // index order follows the memory layout so that consecutive threads touch consecutive addresses
 // index -> (img, ch, y, x) in memory order of the layout; 32-bit arithmetic whenever the index fits (64-bit division is
@@ -423,16 +415,19 @@ __device__ __forceinline__ Vec<CH> ldv(const float* p) {
   if constexpr (CH == 4) {
     const float4 t = __ldg(reinterpret_cast<const float4*>(p));
     r.v[0] = t.x; r.v[1] = t.y; r.v[2] = t.z; r.v[3] = t.w;
-  } else {
+  } else if constexpr (CH == 2) {
     const float2 t = __ldg(reinterpret_cast<const float2*>(p));
     r.v[0] = t.x; r.v[1] = t.y;
+  } else {
+    r.v[0] = __ldg(p);
   }
   return r;
 }
 template <int CH>
 __device__ __forceinline__ void stv(float* p, const Vec<CH>& r) {
   if constexpr (CH == 4) *reinterpret_cast<float4*>(p) = make_float4(r.v[0], r.v[1], r.v[2], r.v[3]);
-  else *reinterpret_cast<float2*>(p) = make_float2(r.v[0], r.v[1]);
+  else if constexpr (CH == 2) *reinterpret_cast<float2*>(p) = make_float2(r.v[0], r.v[1]);
+  else *p = r.v[0];
 }
 template <int CH>
 __device__ __forceinline__ Vec<CH> zerov() {
@@ -819,6 +814,11 @@ __global__ void __launch_bounds__(ROLL_THREADS) dw_wgrad_roll_kernel(DwArgs a, i
   }
 }
 
+int dw_wgrad_finish(const float* part, int64_t total, int kk, int slices, float scale, float* dw, cudaStream_t s) {
+  launch(dw_wgrad_fin_kernel, (unsigned)cdiv(total * 32, 256), 256, 0, s, part, total, kk, slices, scale, dw);
+  return check_launch("dw_wgrad_fin");
+}
+
 static int check_geo(const OmtConvGeo* g, const char* who) {
   OMT_REQUIRE(g && g->groups == g->ci && g->ci == g->co && g->ci >= 1, "%s: depthwise needs groups == ci == co", who);
   OMT_REQUIRE(g->ks >= 1 && g->ks <= 11 && g->stride >= 1 && g->stride <= 4 && g->pad >= 0 && g->pad <= g->ks,
@@ -913,7 +913,12 @@ int omt_dw_fwd(const OmtConvGeo* g, const OmtAct* x, const float* w, const float
   DwArgs a = mk(g, x, y, w, bias, flags);
   bool xn = is_nhwc(x, g->ci, g->ih, g->iw), yn = is_nhwc(y, g->co, g->oh, g->ow);
   int64_t total = (int64_t)g->n * g->co * g->oh * g->ow;
-  if (xn && yn && g->ci % 4 == 0 && aligned16(x->p) && aligned16(y->p) && (!bias || aligned16(bias))) {
+  const bool vec = g->ci % 4 == 0 && aligned16(x->p) && aligned16(y->p) && (!bias || aligned16(bias));
+  // tiles where the 16-byte kernels cannot go (64 x 97 x 56 x 50 5x5: forward 461 -> 170 us, input gradient 946 -> 172; 64 x 130 x 40 x 40
+  // 7x7: 738 -> 141 and 1249 -> 141); where they can, a thread's private ring without barriers is faster (128 x 96 x 56 x 56: 5x5 118
+  // against 136, 3x3 67 against 85)
+  if (xn && yn && !vec && dw_tile_ok(a)) return dw_tile_conv(a, false, false, st(stream));
+  if (xn && yn && vec) {
     if (rows_ok(g)) {
       Scratch sc;
       r = sc.get(nullptr, 0, (size_t)g->ci * g->ks * g->ks * sizeof(float), stream);
@@ -934,7 +939,27 @@ int omt_dw_dgrad(const OmtConvGeo* g, const OmtAct* gy, const float* w, const Om
   OMT_REQUIRE(gy && dx && gy->p && dx->p && w, "omt_dw_dgrad: null pointer");
   DwArgs a = mk(g, gy, dx, w, nullptr, 0);
   int64_t total = (int64_t)g->n * g->ci * g->ih * g->iw;
-  if (g->ci % 4 == 0 && is_nhwc(dx, g->ci, g->ih, g->iw) && is_nhwc(gy, g->ci, g->oh, g->ow) && aligned16(gy->p) && aligned16(dx->p)) {
+  const bool nhwc = is_nhwc(dx, g->ci, g->ih, g->iw) && is_nhwc(gy, g->ci, g->oh, g->ow);
+  const bool vec = g->ci % 4 == 0 && aligned16(gy->p) && aligned16(dx->p);
+  if (nhwc && !vec && g->stride == 1 && g->pad <= g->ks - 1) {
+    // stride 1: the forward kernel over gy with mirrored taps, as below
+    DwArgs f = a;
+    f.ih = g->oh; f.iw = g->ow; f.oh = g->ih; f.ow = g->iw; f.pad = g->ks - 1 - g->pad;
+    if (dw_tile_ok(f)) return dw_tile_conv(f, true, false, st(stream));
+  }
+  if (nhwc && !vec && g->stride == 2 && rows_ok(g)) {
+    Scratch sc;
+    const int kk = g->ks * g->ks;
+    r = sc.get(nullptr, 0, (size_t)g->ci * kk * sizeof(float), stream);
+    if (r) return r;
+    launch(dw_weight_tc_kernel, (unsigned)cdiv((int64_t)g->ci * kk, 256), 256, 0, st(stream), w, (float*)sc.p, g->ci, kk);
+    const unsigned blocks = (unsigned)cdiv((int64_t)g->n * g->ih * cdiv(g->iw, 4) * g->ci, 256);
+    if (g->ks == 3) launch(dw_dgrad_s2_kernel<3, 4, 1>, blocks, 256, 0, st(stream), a, (const float*)sc.p);
+    else if (g->ks == 5) launch(dw_dgrad_s2_kernel<5, 4, 1>, blocks, 256, 0, st(stream), a, (const float*)sc.p);
+    else launch(dw_dgrad_s2_kernel<7, 4, 1>, blocks, 256, 0, st(stream), a, (const float*)sc.p);
+    return check_launch("dw_dgrad_s2_nhwc");
+  }
+  if (nhwc && vec) {
     Scratch sc;
     r = sc.get(nullptr, 0, (size_t)g->ci * g->ks * g->ks * sizeof(float), stream);
     if (r) return r;
@@ -969,16 +994,24 @@ int omt_dw_wgrad(const OmtConvGeo* g, const OmtAct* x, const OmtAct* gy, float* 
   DwArgs a = mk(g, x, gy, nullptr, nullptr, 0);
   cudaStream_t s = st(stream);
   const int c = g->ci, kk = g->ks * g->ks;
+  if (is_nhwc(x, c, g->ih, g->iw) && is_nhwc(gy, c, g->oh, g->ow) && dw_tile_ok(a)) {
+    const bool vec = c % 4 == 0 && aligned16(x->p) && aligned16(gy->p);
+    // tiles, but for the two cases where the 16-byte kernels keep up: 5x5 stride 1 (32 x 240 x 14 x 14 23.6 us against 26.7) and 3x3
+    // stride 2 (32 x 72 x 56 x 56 27.5 against 30.0). Else (old against tiles): 7x7 64 x 96 x 56 x 56 1564 and 122 us; 5x5 stride 2 64 x 96 x
+    // 112 x 112 189 and 131; 3x3 128 x 96 x 56 x 56 91 and 86, 128 x 48 x 7 x 7 19.5 and 13.3; no multiple of four channels, 64 x 97 x 56 x 50
+    // 5x5, 452 and 212
+    if (!vec || g->ks == 7 || (g->ks == 5) == (g->stride == 2) || g->ow <= 8) return dw_tile_wgrad(a, vec, scale, dw, stream);
+  }
   const bool nhwc = is_nhwc(x, c, g->ih, g->iw) && is_nhwc(gy, c, g->oh, g->ow) && c >= 32;
   const bool reg = g->ks == 3 || g->ks == 5 || g->ks == 7;
-  if (is_nhwc(x, c, g->ih, g->iw) && is_nhwc(gy, c, g->oh, g->ow) && c % 4 == 0 && (g->ks == 3 || g->ks == 5) && g->stride <= 2 &&
-      aligned16(x->p) && aligned16(gy->p)) {
+  if (is_nhwc(x, c, g->ih, g->iw) && is_nhwc(gy, c, g->oh, g->ow) && c % 4 == 0 && aligned16(x->p) && aligned16(gy->p) &&
+      ((g->ks == 5 && g->stride == 1) || (g->ks == 3 && g->stride == 2))) {
     float* part = nullptr;
     int S = 1;
     Scratch sc;
     if (g->stride == 1) {
-      // rolling strips; 4 channels per thread for 3x3, 2 for 5x5 (25 tap sums per channel)
-      const int CH = g->ks == 3 ? 4 : 2, TX = 4;
+      // rolling strips; 2 channels per thread (25 tap sums per channel)
+      const int CH = 2, TX = 4;
       const int cqn = c / CH;
       const int CL = std::min(cqn, 32), PL = ROLL_THREADS / CL;
       const int gx = (int)cdiv(cqn, CL);
@@ -992,8 +1025,7 @@ int omt_dw_wgrad(const OmtConvGeo* g, const OmtAct* x, const OmtAct* gy, float* 
       if (r) return r;
       part = (float*)sc.p;
       dim3 grid(gx, S);
-      if (g->ks == 3) launch_wgrad_roll<3, 1, 4, 4>(a, grid, S, CL, rows, segs, part, s);
-      else launch_wgrad_roll<5, 1, 4, 2>(a, grid, S, CL, rows, segs, part, s);
+      launch_wgrad_roll<5, 1, 4, 2>(a, grid, S, CL, rows, segs, part, s);
     } else {  // stride 2: a group of four output pixels per trip (measured 0.77 of the copy bandwidth against 0.61 for strips)
       const int c4 = c / 4;
       const int CL = std::min(c4, 32), PL = 256 / CL;
@@ -1005,8 +1037,7 @@ int omt_dw_wgrad(const OmtConvGeo* g, const OmtAct* x, const OmtAct* gy, float* 
       part = (float*)sc.p;
       dim3 grid(gx, S);
       const size_t smem = (size_t)PL * CL * sizeof(float4);
-      if (g->ks == 3) launch(dw_wgrad_nhwc4_kernel<3, 2>, grid, 256, smem, s, a, S, CL, part);
-      else launch(dw_wgrad_nhwc4_kernel<5, 2>, grid, 256, smem, s, a, S, CL, part);
+      launch(dw_wgrad_nhwc4_kernel<3, 2>, grid, 256, smem, s, a, S, CL, part);
     }
     r = check_launch(g->stride == 1 ? "dw_wgrad_strips_nhwc" : "dw_wgrad_nhwc4");
     if (r) return r;

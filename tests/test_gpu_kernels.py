@@ -916,3 +916,43 @@ def test_add_list(capi, count):
     want = torch.arange(2 * count + 1, dtype=torch.float32)
     want[0:2 * count:2] += 2.5
     assert torch.equal(t.cpu(), want)
+
+
+DW_TILES = [  # n, c, h, w, ks, stride, pad: widths around a group of four and a tile of 64, channels around a slab of 32, short and tall strips, one and several images per block
+    (1, 1, 3, 3, 3, 1, 1), (2, 5, 7, 4, 3, 1, 0), (3, 31, 9, 5, 5, 1, 2), (5, 33, 4, 63, 3, 1, 1), (2, 36, 8, 65, 7, 1, 3), (1, 32, 70, 3, 5, 1, 4), (17, 40, 7, 7, 5, 1, 2),
+    (2, 64, 33, 129, 3, 1, 2), (3, 8, 6, 6, 7, 1, 6), (2, 6, 5, 5, 5, 1, 5), (4, 12, 9, 11, 3, 2, 1), (3, 35, 15, 66, 5, 2, 2), (2, 34, 16, 131, 7, 2, 3), (33, 4, 8, 8, 3, 2, 0), (1, 96, 41, 40, 7, 2, 6),
+]
+
+
+@pytest.mark.parametrize("case", DW_TILES, ids=lambda t: "x".join(map(str, t)))
+def test_depthwise_tiles_vs_aten(capi, case):
+    """Forward (with bias and ReLU), input gradient and weight gradient of channels-last tensors against float64 aten; with 16-byte
+    copies where c % 4 == 0, and again from tensors 4 bytes past a 16-byte boundary. A sum of k products in float32 is within
+    (k + 1) 2^-24 of sum |a b|; that sum comes from the same convolution of the absolute values."""
+    n, c, h, w, ks, s, p = case
+    gen = torch.Generator().manual_seed(sum(case))
+    x, wt, b = torch.randn(n, c, h, w, generator=gen), torch.randn(c, 1, ks, ks, generator=gen), torch.randn(c, generator=gen)
+    xd, wd = x.double().requires_grad_(), wt.double().requires_grad_()
+    y = torch.nn.functional.conv2d(xd, wd, b.double(), s, p, 1, c)
+    gy = torch.randn(y.shape, generator=gen)
+    dx, dw = torch.autograd.grad(y, [xd, wd], gy.double())
+    xa, wa = x.double().abs().requires_grad_(), wt.double().abs().requires_grad_()
+    ya = torch.nn.functional.conv2d(xa, wa, b.double().abs(), s, p, 1, c)
+    dxa, dwa = torch.autograd.grad(ya, [xa, wa], gy.double().abs())
+    eps = 2.0**-24
+
+    def place(t, shift):
+        m, ch, hh, ww = t.shape
+        flat = torch.empty(t.numel() + 1, device="cuda")[shift:shift + t.numel()]
+        v = flat.view(m, hh, ww, ch).permute(0, 3, 1, 2)
+        v.copy_(t)
+        return v
+
+    for shift in (0, 1):
+        xc, gc = place(x, shift), place(gy, shift)
+        got = capi.dw_fwd(xc, wt.cuda(), b.cuda(), s, p, flags=capi.EPI_RELU, cl=True)
+        assert ((got.cpu().double() - y.detach().relu()).abs() <= (ks * ks + 2) * eps * ya.detach() + 1e-30).all()
+        got = capi.dw_dgrad(gc, wt.cuda(), (h, w), s, p, cl=True)
+        assert ((got.cpu().double() - dx).abs() <= (ks * ks + 1) * eps * dxa + 1e-30).all()
+        got = capi.dw_wgrad(xc, gc, ks, s, p, 0.5)
+        assert ((got.cpu().double() - 0.5 * dw).abs() <= (n * y.shape[2] * y.shape[3] + 8) * eps * dwa * 0.5 + 1e-30).all()
