@@ -275,9 +275,9 @@ __global__ void __launch_bounds__(TILE_THREADS, KS == 7 ? 1 : 2) dw_wgrad_tile_k
   }
 }
 
-// Tiles of a layer: up to 16 column groups and as many images as fit 256 threads; then smaller image groups and shorter strips
-// until the launch has `want` blocks (a strip re-reads ks - stride input rows of its upper neighbour: none below ks + 1 rows)
-static TilePlan plan_tiles(const DwArgs& a, int64_t want) {
+// Tiles of a layer: up to 16 column groups and as many images as fit 256 threads; then smaller image groups and strips down to
+// min_rows until the launch has `want` blocks (a strip re-reads ks - stride input rows of its upper neighbour)
+static TilePlan plan_tiles(const DwArgs& a, int64_t want, int min_rows) {
   TilePlan p{};
   const int gx = (int)cdiv(a.ow, TX);
   p.xtiles = (int)cdiv(gx, TILE_THREADS / 16);
@@ -287,7 +287,7 @@ static TilePlan plan_tiles(const DwArgs& a, int64_t want) {
   p.Z = std::max(1, std::min(a.n, TILE_THREADS / (16 * p.G)));
   while (p.Z > 1 && p.Z * p.G * 16 > 64 && per * cdiv(a.n, p.Z) < want) p.Z = (p.Z + 1) / 2;
   p.imgs = (int)cdiv(a.n, p.Z);
-  const int most = std::max(1, a.oh / std::min(a.oh, a.ks + 1));
+  const int most = std::max(1, a.oh / std::min(a.oh, min_rows));
   p.seg_rows = (int)cdiv(a.oh, std::min<int64_t>(std::max<int64_t>(1, cdiv(want, per * p.imgs)), most));
   p.segs = (int)cdiv(a.oh, p.seg_rows);
   return p;
@@ -324,7 +324,7 @@ static void run_conv_ks(const DwArgs& a, const TilePlan& p, bool flip, cudaStrea
   else run_conv<KS, 1, false, VEC>(a, p, s);
 }
 int dw_tile_conv(const DwArgs& a, bool flip, bool vec, cudaStream_t s) {
-  const TilePlan p = plan_tiles(a, (int64_t)8 * sm_count());
+  const TilePlan p = plan_tiles(a, (int64_t)8 * sm_count(), (a.ks + a.stride) / a.stride);  // 8 x 501 x 60 x 60 3x3 stride 2: 55 us with strips twice as tall, 47 so
   if (a.ks == 3) vec ? run_conv_ks<3, 4>(a, p, flip, s) : run_conv_ks<3, 1>(a, p, flip, s);
   else if (a.ks == 5) vec ? run_conv_ks<5, 4>(a, p, flip, s) : run_conv_ks<5, 1>(a, p, flip, s);
   else vec ? run_conv_ks<7, 4>(a, p, flip, s) : run_conv_ks<7, 1>(a, p, flip, s);
@@ -345,7 +345,7 @@ int dw_tile_wgrad(const DwArgs& a, bool vec, float scale, float* dw, omt_stream_
   const int64_t slabs = cdiv(a.c, SLAB);
   const int per_sm = a.ks == 7 ? 1 : 2;
   const int64_t resident = std::max<int64_t>(1, (int64_t)per_sm * sm_count() / slabs);  // blocks per slab that run at once
-  const TilePlan p = plan_tiles(a, 4 * resident * slabs);
+  const TilePlan p = plan_tiles(a, 4 * resident * slabs, a.ks + 1);
   const int SL = (int)std::min<int64_t>(resident, (int64_t)p.imgs * p.segs * p.xtiles);
   const int kk = a.ks * a.ks;
   Scratch sc;
