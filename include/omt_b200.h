@@ -277,6 +277,10 @@ int omt_bn_apply_pool2(const OmtAct* x, const OmtAct* y, const OmtAct* z, uint8_
 int omt_bn_eval(const OmtAct* x, const OmtAct* y, int32_t n, int32_t c, int32_t h, int32_t w, const float* rm,
                 const float* rv, const float* gamma, const float* beta, float eps, uint32_t flags,
                 omt_stream_t stream);
+/* Convolution followed by an eval BatchNorm (folded into the weights and the bias on their way to the GEMM) and, with
+ * OMT_EPI_RELU, a ReLU: conv_bn_act_eval, csrc/fused.cpp:42-49. bias (of the convolution) may be NULL. */
+int omt_conv_fwd_bn(const OmtConvGeo* g, const OmtAct* x, const float* w, const float* bias, const float* gamma, const float* beta,
+                    const float* rm, const float* rv, float eps, const OmtAct* y, uint32_t flags, omt_stream_t stream);
 /* Eval folding (fold_bn, csrc/fused.cpp:34-40; csrc/plans.cpp:148-160): fw[co][k] = w * scale and
  * fb[co] = (bias - rm) * scale + beta with scale = gamma * rsqrt(rv + eps); bias may be NULL (0). k = ci * ks * ks. */
 int omt_bn_fold(const float* w, const float* bias, const float* gamma, const float* beta, const float* rm, const float* rv,

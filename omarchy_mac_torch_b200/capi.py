@@ -106,6 +106,7 @@ SIGNATURES = {
     "omt_bn_apply_add": (_I, [_A, _A, _A, _I, _I, _I, _I, _P, _P, _P, _P, _U, _P]),
     "omt_bn_apply_pool2": (_I, [_A, _A, _A, _P, _I, _I, _I, _I, _P, _P, _P, _P, _U, _P]),
     "omt_bn_eval": (_I, [_A, _A, _I, _I, _I, _I, _P, _P, _P, _P, _F, _U, _P]),
+    "omt_conv_fwd_bn": (_I, [_G, _A, _P, _P, _P, _P, _P, _P, _F, _A, _U, _P]),
     "omt_bn_fold": (_I, [_P, _P, _P, _P, _P, _P, _F, _I, _I, _P, _P, _P]),
     "omt_bn_backward": (_I, [_A, _A, _A, _A, _I, _I, _I, _I, _P, _P, _P, _P, _F, _U, _P]),
     "omt_bn_backward_add": (_I, [_A, _A, _A, _A, _A, _I, _I, _I, _I, _P, _P, _P, _P, _F, _U, _P]),

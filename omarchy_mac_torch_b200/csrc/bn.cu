@@ -602,19 +602,14 @@ static size_t part_floats(int c) { return (size_t)c * (size_t)std::max(8, 4 * sm
 // scale = gamma * rsqrt(var + eps) per output channel. Written as elementwise tensor ops this is seven launches per layer
 // of a few thousand elements each, and the host's ~10 us per op was what an eval pass of a deep network took (ResNet-50,
 // batch 32: 5.2 ms per pass). One launch does all of it; every product and sum is rounded separately, as those ops round.
-__global__ void __launch_bounds__(256) bn_fold_kernel(const float* __restrict__ w, const float* __restrict__ bias, const float* __restrict__ gamma,
-                                                      const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ var,
-                                                      float eps, uint32_t total, uint32_t k, float* __restrict__ fw, float* __restrict__ fb) {
+__global__ void __launch_bounds__(256) bn_fold_kernel(const float* __restrict__ w, const BnFold f, uint32_t total, uint32_t k, float* __restrict__ fw) {
   pdl_wait();
   const uint32_t i = blockIdx.x * 256u + threadIdx.x;
   if (i >= total) return;
   const uint32_t co = i / k;
-  const float scale = __fmul_rn(__ldg(gamma + co), rsqrtf(__fadd_rn(__ldg(var + co), eps)));
+  const float scale = fold_scale(f, co);
   fw[i] = __fmul_rn(__ldg(w + i), scale);
-  if (i == co * k) {
-    const float m = __ldg(mean + co);
-    fb[co] = __fadd_rn(__fmul_rn(bias ? __fsub_rn(__ldg(bias + co), m) : -m, scale), __ldg(beta + co));
-  }
+  if (i == co * k) f.fb[co] = fold_bias(f, co, scale);
 }
 
 }  // namespace omt
@@ -723,7 +718,7 @@ int omt_bn_fold(const float* w, const float* bias, const float* gamma, const flo
                 int32_t co, int32_t k, float* fw, float* fb, omt_stream_t stream) {
   OMT_REQUIRE(w && gamma && beta && rm && rv && fw && fb && co > 0 && k > 0 && (int64_t)co * k < (1ll << 31), "omt_bn_fold: bad arguments");
   const uint32_t total = (uint32_t)co * (uint32_t)k;
-  launch(bn_fold_kernel, (unsigned)cdiv(total, 256), 256, 0, st(stream), w, bias, gamma, beta, rm, rv, eps, total, (uint32_t)k, fw, fb);
+  launch(bn_fold_kernel, (unsigned)cdiv(total, 256), 256, 0, st(stream), w, BnFold{bias, gamma, beta, rm, rv, eps, fb}, total, (uint32_t)k, fw);
   return check_launch("bn_fold");
 }
 

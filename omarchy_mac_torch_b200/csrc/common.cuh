@@ -92,6 +92,9 @@ inline bool is_nhwc(const OmtAct* a, int c, int h, int w) {
 struct PlanOverride { int bn; double mult; };
 extern thread_local PlanOverride tl_plan;
 
+// An eval BatchNorm behind a convolution, folded into its weights and bias: see omt_conv_fwd_bn. `fb` receives the folded bias.
+struct BnFold { const float* bias; const float* gamma; const float* beta; const float* mean; const float* var; float eps; float* fb; };
+
 // Argument checks every dense-convolution entry point starts with (the reference's conv_kind / NEED rules,
 // csrc/conv.cpp:167-183): a square kernel up to 11, stride 1..4, pad <= ks, consistent output size, GEMM extents below 2^31.
 inline int check_dense(const OmtConvGeo* g, const char* who) {
@@ -110,6 +113,12 @@ inline int check_dense(const OmtConvGeo* g, const char* who) {
 }
 
 #ifdef __CUDACC__
+// scale of output channel co, and its folded bias; every product and sum rounded separately, as elementwise tensor ops round them
+__device__ __forceinline__ float fold_scale(const BnFold& f, int co) { return __fmul_rn(__ldg(f.gamma + co), rsqrtf(__fadd_rn(__ldg(f.var + co), f.eps))); }
+__device__ __forceinline__ float fold_bias(const BnFold& f, int co, float scale) {
+  const float m = __ldg(f.mean + co);
+  return __fadd_rn(__fmul_rn(f.bias ? __fsub_rn(__ldg(f.bias + co), m) : -m, scale), __ldg(f.beta + co));
+}
 // Programmatic dependent launch. A training step of a small network is a chain of several hundred kernels of a few
 // microseconds, and between two of them the GPU drains, launches and fills again. Every kernel of the library is launched with
 // programmatic stream serialisation (launch() below; pdl_attr() where a launch has attributes of its own) and starts with

@@ -26,7 +26,7 @@ size_t simt_wgrad_workspace(const OmtConvGeo* g);
 bool tc_supported(int kind, const OmtConvGeo* g, const OmtAct* a, const OmtAct* b);
 size_t tc_workspace(int kind, const OmtConvGeo* g);
 int tc_conv_fwd(const OmtConvGeo* g, const OmtAct* x, const float* w, const float* bias, const OmtAct* y, float* stats,
-                uint32_t flags, void* ws, cudaStream_t s);
+                uint32_t flags, void* ws, cudaStream_t s, const BnFold* fold);
 int tc_conv_dgrad(const OmtConvGeo* g, const OmtAct* gy, const float* w, const OmtAct* dx, uint32_t flags, void* ws, cudaStream_t s);
 int tc_conv_wgrad(const OmtConvGeo* g, const OmtAct* x, const OmtAct* gy, float* dw, float scale, void* ws, cudaStream_t s);
 int tc_bnstats_groups(const OmtConvGeo* g, const OmtAct* x, const OmtAct* y);
@@ -277,8 +277,8 @@ size_t omt_conv_bnstats_floats(int32_t groups, int32_t co) {
   return (size_t)groups * (2 * (size_t)co + 1) + (size_t)cdiv(co, 32);
 }
 
-int omt_conv_fwd(const OmtConvGeo* g, const OmtAct* x, const float* w, const float* bias, const OmtAct* y, float* stats,
-                 uint32_t flags, void* workspace, size_t workspace_bytes, omt_stream_t stream) {
+static int conv_fwd(const OmtConvGeo* g, const OmtAct* x, const float* w, const float* bias, const OmtAct* y, float* stats,
+                 uint32_t flags, void* workspace, size_t workspace_bytes, omt_stream_t stream, BnFold* fold) {
   int r = check_dense(g, "omt_conv_fwd");
   if (r) return r;
   PlanScope plan(0, g);
@@ -299,11 +299,43 @@ int omt_conv_fwd(const OmtConvGeo* g, const OmtAct* x, const float* w, const flo
   }
   OMT_REQUIRE(tc || !(flags & OMT_FORCE_TC), "omt_conv_fwd: geometry/layout not covered by the tensor-core path");
   OMT_REQUIRE(tc || !(flags & OMT_EPI_BNSTATS), "omt_conv_fwd: OMT_EPI_BNSTATS needs the tensor-core path");
+  Scratch fsc;
+  if (fold) {
+    // on the tensor cores the weights are re-laid by a kernel of its own, which folds on the way; elsewhere (and for the first
+    // layers' window mode) they are folded into a copy first
+    const bool own = !tc || g->ci <= 4;
+    const int k = g->ci * g->ks * g->ks;
+    const size_t fbn = (size_t)(g->co + 63) / 64 * 64;
+    r = fsc.get(nullptr, 0, (fbn + (own ? (size_t)g->co * k : 0)) * sizeof(float), stream);
+    if (r) return r;
+    fold->fb = (float*)fsc.p;
+    if (own) {
+      float* fw = fold->fb + fbn;
+      r = omt_bn_fold(w, fold->bias, fold->gamma, fold->beta, fold->mean, fold->var, fold->eps, g->co, k, fw, fold->fb, stream);
+      if (r) return r;
+      w = fw;
+    }
+    bias = fold->fb;
+    flags |= OMT_EPI_BIAS;
+    if (own) fold = nullptr;
+  }
   if (!tc) return simt_conv_fwd(g, x, w, bias, y, flags, st(stream));
   Scratch sc;
   r = sc.get(workspace, workspace_bytes, tc_workspace(0, g), stream);
   if (r) return r;
-  return tc_conv_fwd(g, x, w, bias, y, stats, flags, sc.p, st(stream));
+  return tc_conv_fwd(g, x, w, bias, y, stats, flags, sc.p, st(stream), fold);
+}
+
+int omt_conv_fwd(const OmtConvGeo* g, const OmtAct* x, const float* w, const float* bias, const OmtAct* y, float* stats,
+                 uint32_t flags, void* workspace, size_t workspace_bytes, omt_stream_t stream) {
+  return conv_fwd(g, x, w, bias, y, stats, flags, workspace, workspace_bytes, stream, nullptr);
+}
+
+int omt_conv_fwd_bn(const OmtConvGeo* g, const OmtAct* x, const float* w, const float* bias, const float* gamma, const float* beta,
+                    const float* rm, const float* rv, float eps, const OmtAct* y, uint32_t flags, omt_stream_t stream) {
+  OMT_REQUIRE(gamma && beta && rm && rv && !(flags & ~(uint32_t)OMT_EPI_RELU), "omt_conv_fwd_bn: bad arguments");
+  BnFold f{bias, gamma, beta, rm, rv, eps, nullptr};
+  return conv_fwd(g, x, w, nullptr, y, nullptr, flags, nullptr, 0, stream, &f);
 }
 
 int omt_conv_dgrad(const OmtConvGeo* g, const OmtAct* gy, const float* w, const OmtAct* dx, uint32_t flags, void* workspace,

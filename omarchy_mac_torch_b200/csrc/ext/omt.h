@@ -156,11 +156,15 @@ auto dev_or_composite(const char* name, const A&... a) {
 OmtConvGeo conv_geo(int64_t n, int64_t ci, int64_t co, int64_t ih, int64_t iw, int64_t ks, int64_t stride, int64_t pad,
                     int64_t groups = 1);
 // y = conv(x, w) (+bias)(ReLU) into a fresh tensor; x must be dense4. Output is channels-last when prefer_cl() says so.
+void maybe_tune(int kind, const OmtConvGeo& g);  // the opt-in tuning pass, before a geometry is first used
 Tensor conv_forward(const Tensor& x, const Tensor& w, const Tensor* bias, const OmtConvGeo& g, bool relu);
 bool prefer_cl(const Tensor& x, int64_t co);
 // The same (no ReLU) with the batch-norm partial statistics of y taken in the GEMM epilogue when the call allows it: `groups`
 // is the number of 32-row groups in `partials` (0 and an undefined tensor otherwise; see omt_conv_bnstats_groups).
 Tensor conv_forward_stats(const Tensor& x, const Tensor& w, const Tensor* bias, const OmtConvGeo& g, Tensor& partials, int& groups);
+// conv + eval BatchNorm (+ ReLU) in one call of the library (fused.cpp); an undefined tensor when it does not cover the operands
+Tensor conv_bn_eval(const Tensor& x, const Tensor& cw, const Tensor& cb, const Tensor& w, const Tensor& b, const Tensor& rm, const Tensor& rv, double eps,
+                    const OmtConvGeo& g, bool relu);
 // eval folding of a BatchNorm into the convolution in front of it (fused.cpp): folded weight and bias
 std::pair<Tensor, Tensor> fold_bn_dev(const Tensor& cw, const std::optional<Tensor>& cb, const Tensor& w, const Tensor& b, const Tensor& rm,
                                       const Tensor& rv, double eps);

@@ -137,9 +137,16 @@ static Tensor plan_forward(Plan& p, const Tensor& x_) {
       bool fold = !p.train && g_fold > 0 && li + 1 < p.layers.size() && p.layers[li + 1].kind == "bn";
       if (fold) {
         const Layer& B = p.layers[li + 1];
-        auto f = fold_bn_dev(wt, bias ? std::optional<Tensor>(*bias) : std::nullopt, p.params[B.param], p.params[B.param + 1], p.rms[B.bn], p.rvs[B.bn],
-                             (double)kEps);
-        cur = run_conv(cur, f.first, &f.second, L, true);
+        Tensor y;
+        if (L.is_conv())
+          y = conv_bn_eval(cur, wt, bias ? *bias : Tensor(), p.params[B.param], p.params[B.param + 1], p.rms[B.bn], p.rvs[B.bn], (double)kEps,
+                           conv_geo(cur.size(0), cur.size(1), L.co, cur.size(2), cur.size(3), L.ks, 1, L.ks / 2, 1), true);
+        if (!y.defined()) {
+          auto f = fold_bn_dev(wt, bias ? std::optional<Tensor>(*bias) : std::nullopt, p.params[B.param], p.params[B.param + 1], p.rms[B.bn], p.rvs[B.bn],
+                               (double)kEps);
+          y = run_conv(cur, f.first, &f.second, L, true);
+        }
+        cur = y;
         li++;  // the bn layer is done
       } else if (p.train && L.is_conv() && li + 1 < p.layers.size() && p.layers[li + 1].kind == "bn") {
         // the conv epilogue reduces the BatchNorm's batch statistics while it stores its output

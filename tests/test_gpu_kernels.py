@@ -956,3 +956,43 @@ def test_depthwise_tiles_vs_aten(capi, case):
         assert ((got.cpu().double() - dx).abs() <= (ks * ks + 1) * eps * dxa + 1e-30).all()
         got = capi.dw_wgrad(xc, gc, ks, s, p, 0.5)
         assert ((got.cpu().double() - 0.5 * dw).abs() <= (n * y.shape[2] * y.shape[3] + 8) * eps * dwa * 0.5 + 1e-30).all()
+
+
+@pytest.mark.parametrize("case", [(2, 8, 9, 6, 6, 1, 1, 0), (2, 12, 40, 9, 7, 3, 1, 1), (1, 72, 33, 9, 9, 3, 2, 1), (1, 36, 100, 12, 12, 5, 1, 2), (1, 64, 8, 15, 15, 7, 2, 3), (1, 8, 36, 14, 14, 11, 4, 2), (3, 260, 12, 4, 4, 2, 1, 0),
+                                  (1, 512, 64, 4, 5, 3, 1, 1), (1, 256, 66, 4, 4, 3, 1, 1)], ids=lambda t: "x".join(map(str, t)))
+def test_tensor_core_weights_and_split_reductions(capi, case):
+    """Weight re-layout at every filter size class and ragged channel counts, and split reductions with column counts that are and are
+    not multiples of four: forward and input gradient on the tensor cores against float64 aten (TOL, the path's own bound)."""
+    n, ci, co, h, w, ks, s, p = case
+    gen = torch.Generator().manual_seed(sum(case))
+    x, wt, b = torch.randn(n, ci, h, w, generator=gen), torch.randn(co, ci, ks, ks, generator=gen) / (ci * ks * ks) ** 0.5, torch.randn(co, generator=gen)
+    xd = x.double().requires_grad_()
+    y = torch.nn.functional.conv2d(xd, wt.double(), b.double(), s, p)
+    gy = torch.randn(y.shape, generator=gen)
+    dx, = torch.autograd.grad(y, [xd], gy.double())
+    got = capi.conv_fwd(dev(x, True), wt.cuda(), b.cuda(), s, p, flags=capi.FORCE_TC | capi.EPI_RELU, cl=True)
+    assert rel_err(host(got), y.detach().relu().numpy()) <= TOL
+    if co % 4 == 0:
+        assert rel_err(host(capi.conv_dgrad(dev(gy, True), wt.cuda(), (h, w), s, p, flags=capi.FORCE_TC, cl=True)), dx.numpy()) <= TOL
+
+
+@pytest.mark.parametrize("case", [(2, 8, 12, 9, 7, 3, 1, 1), (1, 36, 100, 12, 12, 1, 2, 0), (3, 3, 64, 30, 30, 7, 2, 3), (2, 5, 9, 8, 8, 3, 1, 1), (2, 64, 66, 10, 10, 5, 1, 2), (1, 256, 64, 4, 4, 3, 1, 1)],
+                         ids=lambda t: "x".join(map(str, t)))
+@pytest.mark.parametrize("bias", [False, True])
+def test_conv_with_a_folded_batch_norm_in_one_call(capi, case, bias):
+    """omt_conv_fwd_bn gives the bits of omt_bn_fold followed by omt_conv_fwd, on the tensor cores (where the weight re-layout folds), in
+    window mode and on the CUDA cores."""
+    n, ci, co, h, w, ks, s, p = case
+    gen = torch.Generator().manual_seed(sum(case))
+    x = dev(torch.randn(n, ci, h, w, generator=gen), ci > 4)
+    wt, cb = torch.randn(co, ci, ks, ks, generator=gen).cuda(), torch.randn(co, generator=gen).cuda()
+    gamma, beta, rm = (torch.randn(co, generator=gen).cuda() for _ in range(3))
+    rv = torch.rand(co, generator=gen).cuda() + 1e-3
+    fw, fb = torch.empty_like(wt), torch.empty_like(cb)
+    q, b_ = capi.ptr, capi.ptr(cb if bias else None)
+    capi.call("omt_bn_fold", q(wt), b_, q(gamma), q(beta), q(rm), q(rv), 1e-5, co, ci * ks * ks, q(fw), q(fb), capi.stream_handle())
+    want = capi.conv_fwd(x, fw, fb, s, p, flags=capi.EPI_RELU, cl=True)
+    got = torch.full_like(want, float("nan"))
+    g = capi.geo(n, ci, co, h, w, ks, s, p)
+    capi.call("omt_conv_fwd_bn", g, capi.act(x), q(wt), b_, q(gamma), q(beta), q(rm), q(rv), 1e-5, capi.act(got), capi.EPI_RELU, capi.stream_handle())
+    assert torch.equal(got, want)
