@@ -996,3 +996,17 @@ def test_conv_with_a_folded_batch_norm_in_one_call(capi, case, bias):
     g = capi.geo(n, ci, co, h, w, ks, s, p)
     capi.call("omt_conv_fwd_bn", g, capi.act(x), q(wt), b_, q(gamma), q(beta), q(rm), q(rv), 1e-5, capi.act(got), capi.EPI_RELU, capi.stream_handle())
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("shape", [(1, 4, 2, 2), (2, 8, 5, 7), (3, 36, 6, 3), (16, 64, 9, 16), (1, 1028, 4, 5)], ids=lambda s: "x".join(map(str, s)))
+def test_pool2_backward_of_channels_last_tensors(capi, shape):
+    """Four channels of a 2x2 block per thread gives what one element per thread gives (the NCHW kernel), odd sizes and ties included."""
+    n, c, h, w = shape
+    gen = torch.Generator().manual_seed(c)
+    x = torch.randint(0, 3, shape, generator=gen).float()
+    gy = torch.randn(n, c, h // 2, w // 2, generator=gen)
+    _, i0 = capi.pool2_fwd(dev(x))
+    _, i1 = capi.pool2_fwd(dev(x, True))
+    assert torch.equal(i0.cpu(), i1.cpu())
+    want, got = capi.pool2_bwd(dev(gy), i0, (h, w)), capi.pool2_bwd(dev(gy, True), i1, (h, w))
+    assert torch.equal(got.cpu(), want.cpu()) and torch.count_nonzero(want) == gy.numel()
