@@ -198,6 +198,10 @@ int omt_conv_wgrad_noalloc(const OmtConvGeo* g, const OmtAct* x, const OmtAct* g
 /* db[c] = sum over (n,h,w) of gy. Replaces csrc/kernels/csum_nchw.wgsl (csrc/conv.cpp:232-235). */
 int omt_conv_bias_grad(const OmtAct* gy, int32_t n, int32_t c, int32_t h, int32_t w, float* db, float scale,
                        omt_stream_t stream);
+/* out[image][c] = the sum (mean != 0: the mean) over the image's pixels of channels-last images [images][pixels][c]: global
+ * average pooling, its broadcast's gradient, and the bias gradient of a Linear layer (one image of `rows` pixels). The
+ * reference reduces these with its generic kernels (csrc/reduce.cpp:1-127). */
+int omt_channel_sum(const float* x, int32_t images, int64_t pixels, int32_t c, int32_t mean, float* out, omt_stream_t stream);
 
 /* out[M,N] (row-major) = A[M,K] * B[K,N] (+ bias[N]) in float32 on the same tensor-core kernels: a matrix product is the
  * 1x1 case of the implicit GEMM (rows = pixels). Replaces mm_into / mm_ / addmm_ (csrc/linalg.cpp:25-92; the generated

@@ -82,6 +82,7 @@ SIGNATURES = {
     "omt_conv_wgrad_noalloc_capacity": (_SZ, []),
     "omt_conv_wgrad_noalloc": (_I, [_G, _A, _A, _P, _F, _P]),
     "omt_conv_bias_grad": (_I, [_A, _I, _I, _I, _I, _P, _F, _P]),
+    "omt_channel_sum": (_I, [_P, _I, _I64, _I, _I, _P, _P]),
     "omt_kernel_timing": (_I, [_I]),
     "omt_kernel_times": (_SZ, [C.c_char_p, _SZ, _I]),
     "omt_gemm": (_I, [_P, _I64, _I64, _P, _I64, _I64, _P, _P, _I, _I, _I, _P]),

@@ -754,9 +754,11 @@ __global__ void csum_fin_kernel(const float* part, int c, int S, float scale, fl
 // channel walking pixels (what this replaces) left most of the block idle below 256 channels and had one load in flight: with its
 // second launch 74 us for 16 x 64 x 55 x 55 (12 MB), and a PlainCNN step with three such layers went from 568 to 438 us. With one slice the sums are final, else csum_nhwc_fin_kernel adds the slices.
 template <int VEC>
-__global__ void __launch_bounds__(256) csum_nhwc_kernel(const float* __restrict__ gy, int64_t pixels, int c, int CL, int64_t per, float scale,
-                                                        float* __restrict__ out) {  // out[slice][c]
+__global__ void __launch_bounds__(256) csum_nhwc_kernel(const float* __restrict__ gy, int64_t pixels, int c, int CL, int64_t per, float scale, float div,
+                                                        float* __restrict__ out) {  // out[image][slice][c], images of `pixels` pixels each
   pdl_wait();
+  gy += (int64_t)blockIdx.z * pixels * c;
+  out += (int64_t)blockIdx.z * gridDim.y * c;
   __shared__ float red[256][VEC];
   const int PL = 256 / CL, cl = threadIdx.x % CL, pl = threadIdx.x / CL;
   const int ch = ((int)blockIdx.x * CL + cl) * VEC;
@@ -797,12 +799,14 @@ __global__ void __launch_bounds__(256) csum_nhwc_kernel(const float* __restrict_
   }
   if (pl == 0 && live) {
 #pragma unroll
-    for (int e = 0; e < VEC; e++) out[(int64_t)blockIdx.y * c + ch + e] = red[threadIdx.x][e] * scale;
+    for (int e = 0; e < VEC; e++) out[(int64_t)blockIdx.y * c + ch + e] = red[threadIdx.x][e] * scale / div;
   }
 }
 // 32 channels x 16 slice lanes per block
-__global__ void __launch_bounds__(512) csum_nhwc_fin_kernel(const float* __restrict__ part, int c, int S, float scale, float* __restrict__ out) {
+__global__ void __launch_bounds__(512) csum_nhwc_fin_kernel(const float* __restrict__ part, int c, int S, float scale, float div, float* __restrict__ out) {
   pdl_wait();
+  part += (int64_t)blockIdx.y * S * c;
+  out += (int64_t)blockIdx.y * c;
   __shared__ float red[16][33];
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5, ch = blockIdx.x * 32 + x;
   float s = 0.f;
@@ -814,8 +818,32 @@ __global__ void __launch_bounds__(512) csum_nhwc_fin_kernel(const float* __restr
   __syncthreads();
   if (y == 0 && ch < c) {
     for (int k = 1; k < 16; k++) s += red[k][x];
-    out[ch] = s * scale;
+    out[ch] = s * scale / div;
   }
+}
+// out[image][ch] = scale / div * sum over the image's pixels, for images of channels-last pixels
+static int csum_nhwc(const float* x, int64_t images, int64_t pixels, int c, float scale, float div, float* out, omt_stream_t stream) {
+  cudaStream_t s = st(stream);
+  const bool vec = c % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  const int groups = vec ? c / 4 : c, CL = groups <= 64 ? groups : 32;
+  const int64_t gx = cdiv(groups, CL);
+  // slices of 32 KB and more, at most about four blocks per SM
+  const int64_t want = std::min<int64_t>(pixels * c * 4 / gx / (32 << 10), 4 * sm_count() / (gx * images));
+  const int64_t per = cdiv(pixels, std::max<int64_t>(1, want)), S = cdiv(pixels, per);
+  Scratch sc;
+  if (S > 1) {
+    int r = sc.get(nullptr, 0, (size_t)images * c * S * sizeof(float), stream);
+    if (r) return r;
+  }
+  float* part = S > 1 ? (float*)sc.p : out;
+  const float sc1 = S > 1 ? 1.f : scale, dv1 = S > 1 ? 1.f : div;
+  const dim3 grid((unsigned)gx, (unsigned)S, (unsigned)images);
+  if (vec) launch(csum_nhwc_kernel<4>, grid, 256, 0, s, x, pixels, c, CL, per, sc1, dv1, part);
+  else launch(csum_nhwc_kernel<1>, grid, 256, 0, s, x, pixels, c, CL, per, sc1, dv1, part);
+  int r = check_launch("channel_sum_nhwc");
+  if (r || S == 1) return r;
+  launch(csum_nhwc_fin_kernel, dim3((unsigned)cdiv(c, 32), (unsigned)images), 512, 0, s, part, c, (int)S, scale, div, out);
+  return check_launch("channel_sum_nhwc_fin");
 }
 
 }  // namespace omt
@@ -826,28 +854,7 @@ extern "C" int omt_conv_bias_grad(const OmtAct* gy, int32_t n, int32_t c, int32_
                                   omt_stream_t stream) {
   OMT_REQUIRE(gy && gy->p && db && n > 0 && c > 0 && h > 0 && w > 0, "omt_conv_bias_grad: bad arguments");
   cudaStream_t s = st(stream);
-  if (is_nhwc(gy, c, h, w) && c > 1) {
-    const int64_t pixels = (int64_t)n * h * w;
-    const bool vec = c % 4 == 0 && (reinterpret_cast<uintptr_t>(gy->p) & 15) == 0;
-    const int groups = vec ? c / 4 : c, CL = groups <= 64 ? groups : 32;
-    const int64_t gx = cdiv(groups, CL);
-    // slices of 32 KB and more, at most about four blocks per SM
-    const int64_t want = std::min<int64_t>(pixels * c * 4 / gx / (32 << 10), 4 * sm_count() / gx);
-    const int64_t per = cdiv(pixels, std::max<int64_t>(1, want)), S = cdiv(pixels, per);
-    Scratch sc;
-    if (S > 1) {
-      int r = sc.get(nullptr, 0, (size_t)c * S * sizeof(float), stream);
-      if (r) return r;
-    }
-    float* part = S > 1 ? (float*)sc.p : db;
-    const dim3 grid((unsigned)gx, (unsigned)S);
-    if (vec) launch(csum_nhwc_kernel<4>, grid, 256, 0, s, gy->p, pixels, c, CL, per, S > 1 ? 1.f : scale, part);
-    else launch(csum_nhwc_kernel<1>, grid, 256, 0, s, gy->p, pixels, c, CL, per, S > 1 ? 1.f : scale, part);
-    int r = check_launch("bias_grad_nhwc");
-    if (r || S == 1) return r;
-    launch(csum_nhwc_fin_kernel, (unsigned)cdiv(c, 32), 512, 0, s, part, c, (int)S, scale, db);
-    return check_launch("bias_grad_nhwc_fin");
-  }
+  if (is_nhwc(gy, c, h, w) && c > 1) return csum_nhwc(gy->p, 1, (int64_t)n * h * w, c, scale, 1.f, db, stream);
   const int S = (int)std::min<int64_t>(n, std::max<int64_t>(1, (4 * sm_count()) / c));
   Scratch sc;
   int r = sc.get(nullptr, 0, (size_t)c * S * sizeof(float), stream);
@@ -858,4 +865,9 @@ extern "C" int omt_conv_bias_grad(const OmtAct* gy, int32_t n, int32_t c, int32_
   if (r) return r;
   launch(csum_fin_kernel, (unsigned)cdiv(c, 128), 128, 0, s, part, c, S, scale, db);
   return check_launch("bias_grad_fin");
+}
+
+extern "C" int omt_channel_sum(const float* x, int32_t images, int64_t pixels, int32_t c, int32_t mean, float* out, omt_stream_t stream) {
+  OMT_REQUIRE(x && out && images > 0 && images <= 65535 && pixels > 0 && c > 0, "omt_channel_sum: bad arguments");
+  return csum_nhwc(x, images, pixels, c, 1.f, mean ? (float)pixels : 1.f, out, stream);
 }

@@ -149,6 +149,10 @@ static Tensor adaptive_avg_pool2d_(const Tensor& x_, IntArrayRef os) {
   NEED(f32(x_) && x_.dim() == 4 && x_.numel() > 0 && os[0] > 0 && os[1] > 0, "adaptive avg pool: 4-D float32");
   Tensor x = dense4(x_);
   Tensor out = dense4(empty_dev({x.size(0), x.size(1), os[0], os[1]}, at::kFloat, is_cl(x) && os[0] * os[1] > 1));
+  if (os[0] * os[1] == 1 && layout4(x) == 1 && x.size(0) <= 65535) {
+    check(omt_channel_sum(fptr(x), (int)x.size(0), x.size(2) * x.size(3), (int)x.size(1), 1, out.data_ptr<float>(), cur_stream()), "global avg pool");
+    return out;
+  }
   OmtAct ax = act(x), ay = act(out);
   check(omt_adaptive_avgpool_fwd(&ax, &ay, (int)x.size(0), (int)x.size(1), (int)x.size(2), (int)x.size(3), (int)os[0], (int)os[1], cur_stream()),
         "adaptive avg pool");
@@ -163,6 +167,38 @@ static Tensor adaptive_avg_pool2d_backward_(const Tensor& gy_, const Tensor& x) 
                                  cur_stream()),
         "adaptive avg pool backward");
   return gx;
+}
+
+// Sums and means over the pixels of channels-last images (global pooling in eager code is a mean, the gradient of a per-channel
+// gate a sum) and over the rows of a matrix (the bias gradient of nn.Linear) are channel sums; every other reduction goes to
+// ATen's CUDA kernel over the bridge, as all of them did. A MobileNetV3 step has 21 of them
+// of about 12 us in ATen's kernel, for a few hundred KB each: 3632 -> 3575 us.
+static bool channel_sum(const Tensor& x, at::OptionalIntArrayRef dim, bool keepdim, std::optional<at::ScalarType> dtype, bool mean, Tensor& out) {
+  if (!f32(x) || (dtype && *dtype != at::kFloat) || !dim || x.numel() == 0 || x.numel() >= (1ll << 40)) return false;
+  const int64_t R = x.dim();
+  auto wrapped = [&](size_t k) { return (*dim)[k] < 0 ? (*dim)[k] + R : (*dim)[k]; };
+  if (R == 2 && dim->size() == 1 && wrapped(0) == 0 && x.is_contiguous() && x.size(0) > 1 && x.size(1) < (1ll << 31)) {
+    out = keepdim ? empty_dev({1, x.size(1)}, at::kFloat) : empty_dev({x.size(1)}, at::kFloat);
+    check(omt_channel_sum(fptr(x), 1, x.size(0), (int)x.size(1), mean, out.data_ptr<float>(), cur_stream()), "sum over rows");
+    return true;
+  }
+  if (R == 4 && dim->size() == 2 && wrapped(0) + wrapped(1) == 5 && (wrapped(0) == 2 || wrapped(0) == 3) && layout4(x) == 1 && x.size(0) <= 65535 &&
+      x.size(1) < (1ll << 31)) {
+    out = keepdim ? empty_dev({x.size(0), x.size(1), 1, 1}, at::kFloat) : empty_dev({x.size(0), x.size(1)}, at::kFloat);
+    check(omt_channel_sum(fptr(x), (int)x.size(0), x.size(2) * x.size(3), (int)x.size(1), mean, out.data_ptr<float>(), cur_stream()), "sum over pixels");
+    return true;
+  }
+  return false;
+}
+static Tensor sum_dim(const Tensor& x, at::OptionalIntArrayRef dim, bool keepdim, std::optional<at::ScalarType> dtype) {
+  Tensor out;
+  if (channel_sum(x, dim, keepdim, dtype, false, out)) return out;
+  return at::native::call_fallback_fn<&bridge_boxed, at::_ops::sum_dim_IntList>::call(x, dim, keepdim, dtype);
+}
+static Tensor mean_dim(const Tensor& x, at::OptionalIntArrayRef dim, bool keepdim, std::optional<at::ScalarType> dtype) {
+  Tensor out;
+  if (channel_sum(x, dim, keepdim, dtype, true, out)) return out;
+  return at::native::call_fallback_fn<&bridge_boxed, at::_ops::mean_dim>::call(x, dim, keepdim, dtype);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -194,6 +230,8 @@ TORCH_LIBRARY_IMPL(aten, PrivateUse1, m) {
   OMT_IMPL(m, avg_pool2d_backward, avg_pool2d_backward_);
   OMT_IMPL(m, _adaptive_avg_pool2d, adaptive_avg_pool2d_);
   OMT_IMPL(m, _adaptive_avg_pool2d_backward, adaptive_avg_pool2d_backward_);
+  OMT_IMPL(m, sum_dim_IntList, sum_dim);
+  OMT_IMPL(m, mean_dim, mean_dim);
   OMT_IMPL(m, uniform_, uniform_);
   OMT_IMPL(m, normal_, normal_);
 }

@@ -215,8 +215,12 @@ static Tensor plan_forward(Plan& p, const Tensor& x_) {
       cur = y;
     } else {  // gap
       Tensor y = empty_dev({n, c, 1, 1}, at::kFloat);
-      OmtAct ax = act(cur), ay = act(y);
-      check(omt_adaptive_avgpool_fwd(&ax, &ay, n, c, h, w, 1, 1, cur_stream()), "plan global avg pool");
+      if (layout4(cur) == 1 && n <= 65535) {
+        check(omt_channel_sum(fptr(cur), n, (int64_t)h * w, c, 1, y.data_ptr<float>(), cur_stream()), "plan global avg pool");
+      } else {
+        OmtAct ax = act(cur), ay = act(y);
+        check(omt_adaptive_avgpool_fwd(&ax, &ay, n, c, h, w, 1, 1, cur_stream()), "plan global avg pool");
+      }
       cur = y;
     }
   }

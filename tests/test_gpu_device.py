@@ -845,3 +845,33 @@ def test_fused_pointwise_four_elements_at_a_time(omt):
                 whole.append(view(c, 0))
             assert torch.equal(fp(prog, whole).cpu(), fp(prog, shifted).cpu()), (shape, prog)
     assert not omt.FALLBACKS, dict(omt.FALLBACKS)
+
+
+@pytest.mark.parametrize("shape", [(1, 3, 2, 2), (2, 64, 7, 7), (5, 66, 13, 1), (3, 96, 40, 41), (1, 16, 150, 150), (40, 1030, 3, 3)], ids=lambda s: "x".join(map(str, s)))
+def test_channel_sums_serve_sum_mean_and_global_pooling(omt, shape):
+    """sum / mean over the pixels and adaptive pooling to 1x1 of channels-last tensors, sum / mean over a matrix's rows: values against
+    float64 (a float32 sum of k terms is within k 2^-24 of sum |x|; lanes add at most k / 256 in a row), shapes, strides and the
+    forms that stay with ATen."""
+    n, c, h, w = shape
+    x = torch.randn(shape).contiguous(memory_format=torch.channels_last)
+    d = x.to(D).contiguous(memory_format=torch.channels_last)
+    eps = (h * w / 256 + 64) * 2.0**-24
+    omt.FALLBACKS.clear()
+    for fn in (torch.sum, torch.mean):
+        for dims in ((2, 3), (-1, -2), (3, 2)):
+            for keep in (False, True):
+                got, want = fn(d, dims, keep), fn(x.double(), dims, keep)
+                assert got.shape == want.shape and got.stride() == fn(x, dims, keep).stride()
+                assert ((got.cpu().double() - want).abs() <= eps * fn(x.double().abs(), dims, keep)).all()
+        for dims, keep in (((0, 1), False), ((1,), True), ((0, 2, 3), False), ((2,), False)):  # ATen's
+            assert e(fn(d, dims, keep), fn(x, dims, keep)) <= 1e-5
+        m = x.permute(0, 2, 3, 1).reshape(-1, c)
+        for keep in (False, True):
+            got, want = fn(m.to(D), 0, keep), fn(m.double(), 0, keep)
+            assert got.shape == want.shape
+            assert ((got.cpu().double() - want).abs() <= (n * h * w / 256 + 64) * 2.0**-24 * fn(m.double().abs(), 0, keep)).all()
+        assert e(fn(m.to(D), 1), fn(m, 1)) <= 1e-5 and e(fn(m.to(D).t(), 0), fn(m.t(), 0)) <= 1e-5
+    assert torch.sum(d, (2, 3), dtype=torch.float64).dtype == torch.float64
+    got = F.adaptive_avg_pool2d(d, 1)
+    assert ((got.cpu().double() - x.double().mean((2, 3), True)).abs() <= eps * x.double().abs().mean((2, 3), True)).all()
+    assert not omt.FALLBACKS, dict(omt.FALLBACKS)
