@@ -346,7 +346,8 @@ int dw_tile_wgrad(const DwArgs& a, bool vec, float scale, float* dw, omt_stream_
   const int per_sm = a.ks == 7 ? 1 : 2;
   const int64_t resident = std::max<int64_t>(1, (int64_t)per_sm * sm_count() / slabs);  // blocks per slab that run at once
   const TilePlan p = plan_tiles(a, 4 * resident * slabs, a.ks + 1);
-  const int SL = (int)std::min<int64_t>(resident, (int64_t)p.imgs * p.segs * p.xtiles);
+  const int64_t small = std::max<int64_t>(1, std::min<int64_t>(4, TILE_THREADS / (16 * p.G * p.Z)));  // blocks of few threads: more per SM (27 x 301 x 23 x 21 7x7 stride 2 110 -> 63 us, 64 x 96 x 56 x 56 77 -> 52)
+  const int SL = (int)std::min<int64_t>(resident * small, (int64_t)p.imgs * p.segs * p.xtiles);
   const int kk = a.ks * a.ks;
   Scratch sc;
   int r = sc.get(nullptr, 0, (size_t)a.c * SL * kk * sizeof(float), stream);
