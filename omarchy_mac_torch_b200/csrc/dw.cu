@@ -939,7 +939,7 @@ int omt_dw_fwd(const OmtConvGeo* g, const OmtAct* x, const float* w, const float
   // tiles where the 16-byte kernels cannot go (64 x 97 x 56 x 50 5x5: forward 461 -> 170 us, input gradient 946 -> 172; 64 x 130 x 40 x 40
   // 7x7: 738 -> 141 and 1249 -> 141); where they can, a thread's private ring without barriers is faster (128 x 96 x 56 x 56: 5x5 118
   // against 136, 3x3 67 against 85)
-  if (xn && yn && !vec && dw_tile_ok(a)) return dw_tile_conv(a, false, false, st(stream));
+  if (xn && yn && !vec && dw_tile_ok(a)) return dw_tile_conv(a, false, st(stream));
   if (xn && yn && vec) {
     if (rows_ok(g)) {
       Scratch sc;
@@ -967,7 +967,7 @@ int omt_dw_dgrad(const OmtConvGeo* g, const OmtAct* gy, const float* w, const Om
     // stride 1: the forward kernel over gy with mirrored taps, as below
     DwArgs f = a;
     f.ih = g->oh; f.iw = g->ow; f.oh = g->ih; f.ow = g->iw; f.pad = g->ks - 1 - g->pad;
-    if (dw_tile_ok(f)) return dw_tile_conv(f, true, false, st(stream));
+    if (dw_tile_ok(f)) return dw_tile_conv(f, true, st(stream));
   }
   if (nhwc && !vec && g->stride == 2 && rows_ok(g)) {
     Scratch sc;

@@ -62,7 +62,7 @@ struct TilePlan {
 };
 
 // Forward (FLIP = false) and stride-1 input gradient (FLIP = true: taps mirrored, pad = ks-1-pad, the caller swaps the tensors).
-template <int KS, int S, bool FLIP, int VEC>
+template <int KS, int S, bool FLIP>
 __global__ void __launch_bounds__(TILE_THREADS, KS == 3 ? 3 : 2) dw_tile_kernel(DwArgs a, TilePlan p) {
   pdl_wait();
   constexpr int SPAN = (TX - 1) * S + KS, R = (KS + S - 1) / S, U = R * S, KK = KS * KS;
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(TILE_THREADS, KS == 3 ? 3 : 2) dw_tile_kernel(
   auto valid = [&](int r) { return img_ok && r < n_in && (unsigned)(sy0 + r) < (unsigned)a.ih; };
   uint32_t wr = 0, rd = 0;  // byte offsets of the slots written and read next
   auto request = [&](int r) {
-    if (valid(r)) copy_row<VEC>(ring + wr, xbase + r * rs, a.x.p, t, nt, cols, x0, a.iw, a.c, ch0);
+    if (valid(r)) copy_row<1>(ring + wr, xbase + r * rs, a.x.p, t, nt, cols, x0, a.iw, a.c, ch0);
     commit();
     wr += slot_bytes;
     if (wr == DEPTH * slot_bytes) wr = 0;
@@ -156,12 +156,8 @@ __global__ void __launch_bounds__(TILE_THREADS, KS == 3 ? 3 : 2) dw_tile_kernel(
               float2 o = unpack2(acc[slot][j]);
               o.x += b0; o.y += b1;
               if (relu) { o.x = fmaxf(o.x, 0.f); o.y = fmaxf(o.y, 0.f); }
-              if constexpr (VEC == 4) {
-                if (ch < a.c) *reinterpret_cast<float2*>(yp + (int64_t)j * a.c) = o;
-              } else {
-                if (ch < a.c) yp[(int64_t)j * a.c] = o.x;
-                if (ch + 1 < a.c) yp[(int64_t)j * a.c + 1] = o.y;
-              }
+              if (ch < a.c) yp[(int64_t)j * a.c] = o.x;
+              if (ch + 1 < a.c) yp[(int64_t)j * a.c + 1] = o.y;
             }
             acc[slot][j] = 0;
           }
@@ -312,22 +308,22 @@ static void allow_smem() {
     if (cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_SMEM_MAX) != cudaSuccess) cudaGetLastError();  // (the launch reports it)
   });
 }
-template <int KS, int S, bool FLIP, int VEC>
+template <int KS, int S, bool FLIP>
 static void run_conv(const DwArgs& a, const TilePlan& p, cudaStream_t s) {
-  allow_smem<dw_tile_kernel<KS, S, FLIP, VEC>>();
-  launch(dw_tile_kernel<KS, S, FLIP, VEC>, (unsigned)(cdiv(a.c, SLAB) * p.xtiles * p.segs * p.imgs), dim3(16 * p.G, p.Z), tile_smem(a, p, false), s, a, p);
+  allow_smem<dw_tile_kernel<KS, S, FLIP>>();
+  launch(dw_tile_kernel<KS, S, FLIP>, (unsigned)(cdiv(a.c, SLAB) * p.xtiles * p.segs * p.imgs), dim3(16 * p.G, p.Z), tile_smem(a, p, false), s, a, p);
 }
-template <int KS, int VEC>
+template <int KS>
 static void run_conv_ks(const DwArgs& a, const TilePlan& p, bool flip, cudaStream_t s) {
-  if (a.stride == 2) run_conv<KS, 2, false, VEC>(a, p, s);
-  else if (flip) run_conv<KS, 1, true, VEC>(a, p, s);
-  else run_conv<KS, 1, false, VEC>(a, p, s);
+  if (a.stride == 2) run_conv<KS, 2, false>(a, p, s);
+  else if (flip) run_conv<KS, 1, true>(a, p, s);
+  else run_conv<KS, 1, false>(a, p, s);
 }
-int dw_tile_conv(const DwArgs& a, bool flip, bool vec, cudaStream_t s) {
+int dw_tile_conv(const DwArgs& a, bool flip, cudaStream_t s) {
   const TilePlan p = plan_tiles(a, (int64_t)8 * sm_count(), (a.ks + a.stride) / a.stride);  // 8 x 501 x 60 x 60 3x3 stride 2: 55 us with strips twice as tall, 47 so
-  if (a.ks == 3) vec ? run_conv_ks<3, 4>(a, p, flip, s) : run_conv_ks<3, 1>(a, p, flip, s);
-  else if (a.ks == 5) vec ? run_conv_ks<5, 4>(a, p, flip, s) : run_conv_ks<5, 1>(a, p, flip, s);
-  else vec ? run_conv_ks<7, 4>(a, p, flip, s) : run_conv_ks<7, 1>(a, p, flip, s);
+  if (a.ks == 3) run_conv_ks<3>(a, p, flip, s);
+  else if (a.ks == 5) run_conv_ks<5>(a, p, flip, s);
+  else run_conv_ks<7>(a, p, flip, s);
   return check_launch(flip ? "dw_dgrad_tile" : "dw_fwd_tile");
 }
 
