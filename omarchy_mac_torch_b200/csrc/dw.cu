@@ -699,9 +699,11 @@ __global__ void __launch_bounds__(256) dw_dgrad_s2_kernel(DwArgs a, const float*
       for (int j = 0; j < TX; j++) {
 #pragma unroll
         for (int m = 0; m <= HALF; m++) {
-          const int kx = ((PE + j) & 1) + 2 * m;
+          const int kx = ((PE + j) & 1) + 2 * m, k = HALF + ((PE + j) >> 1) - m;
           if (kx >= KS) continue;
-          fmav<CH>(acc[j], g[HALF + ((PE + j) >> 1) - m], ldv<CH>(wr + kx * a.c));
+          // one channel per thread: as dw_dgrad_kernel, whose cases these are, leave out the pixels outside (an infinite tap times a zero is no zero)
+          if (CH == 1 && !interior && (unsigned)(ox_base + k) >= (unsigned)a.ow) continue;
+          fmav<CH>(acc[j], g[k], ldv<CH>(wr + kx * a.c));
         }
       }
     };

@@ -33,6 +33,7 @@ __device__ __forceinline__ float2 unpack2(u64 v) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
   return r;
 }
+__device__ __forceinline__ bool finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
 __host__ __device__ constexpr int fdiv(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 __host__ __device__ constexpr int pmod(int a, int b) { return ((a % b) + b) % b; }
 
@@ -61,12 +62,62 @@ struct TilePlan {
   int imgs;            // image groups
 };
 
+// Zeros stand for the pixels outside the image, and zero times infinity is not zero. Only pixels inside the image have a part in a
+// result, so the kernels below fall back to the two functions here, which skip the others, where a non-finite value would meet one of
+// those zeros: a block whose filters are not all finite, and a tap sum that is not finite. (That covers every such product, and a
+// finite run never gets here.)
+template <int KS, int S>
+__device__ __forceinline__ void direct_outputs(const DwArgs& a, const TilePlan& p, const float* ws) {
+  const int slabs = (a.c + SLAB - 1) / SLAB, cols = p.G * TX;
+  int b = blockIdx.x;
+  const int ch0 = (b % slabs) * SLAB; b /= slabs;
+  const int tile0 = b % p.xtiles * cols; b /= p.xtiles;
+  const int oy0 = b % p.segs * p.seg_rows, img = b / p.segs * p.Z + threadIdx.y, nrows = min(p.seg_rows, a.oh - oy0);
+  if (img >= a.n) return;
+  const float* x = a.x.p + (int64_t)img * a.ih * a.iw * a.c;
+  float* y = a.y.p + (int64_t)img * a.oh * a.ow * a.c;
+  for (int e = threadIdx.x; e < nrows * cols * SLAB; e += blockDim.x) {
+    const int cc = e % SLAB, k = e / SLAB, ox = tile0 + k % cols, oy = oy0 + k / cols, ch = ch0 + cc;
+    if (ch >= a.c || ox >= a.ow) continue;
+    float s = 0.f;
+    for (int ky = 0; ky < KS; ky++)
+      for (int kx = 0; kx < KS; kx++) {
+        const int sy = oy * S - a.pad + ky, sx = ox * S - a.pad + kx;
+        if ((unsigned)sy < (unsigned)a.ih && (unsigned)sx < (unsigned)a.iw) s = fmaf(__ldg(x + ((int64_t)sy * a.iw + sx) * a.c + ch), ws[(ky * KS + kx) * SLAB + cc], s);
+      }
+    if (a.flags & OMT_EPI_BIAS) s += __ldg(a.bias + ch);
+    if (a.flags & OMT_EPI_RELU) s = fmaxf(s, 0.f);
+    y[((int64_t)oy * a.ow + ox) * a.c + ch] = s;
+  }
+}
+// the sum of tap (ky, kx) of channel ch over the strips of weight-gradient block sl; ends at the first NaN, which stays one
+template <int S>
+__device__ __forceinline__ float direct_tap_sum(const DwArgs& a, const TilePlan& p, int sl, int SL, int ch, int ky, int kx) {
+  float s = 0.f;
+  for (int it = sl; it < p.imgs * p.segs * p.xtiles; it += SL) {
+    const int tile0 = it % p.xtiles * p.G * TX, q = it / p.xtiles, oy0 = q % p.segs * p.seg_rows, img0 = q / p.segs * p.Z;
+    for (int img = img0; img < min(img0 + p.Z, a.n); img++)
+      for (int oy = oy0; oy < min(oy0 + p.seg_rows, a.oh); oy++) {
+        const int sy = oy * S - a.pad + ky;
+        if ((unsigned)sy >= (unsigned)a.ih) continue;
+        const float* g = a.y.p + ((int64_t)img * a.oh + oy) * a.ow * a.c + ch;
+        const float* x = a.x.p + ((int64_t)img * a.ih + sy) * a.iw * a.c + ch;
+        for (int ox = tile0; ox < min(tile0 + p.G * TX, a.ow); ox++) {
+          const int sx = ox * S - a.pad + kx;
+          if ((unsigned)sx < (unsigned)a.iw) s = fmaf(__ldg(g + (int64_t)ox * a.c), __ldg(x + (int64_t)sx * a.c), s);
+        }
+        if (s != s) return s;
+      }
+  }
+  return s;
+}
+
 // Forward (FLIP = false) and stride-1 input gradient (FLIP = true: taps mirrored, pad = ks-1-pad, the caller swaps the tensors).
 template <int KS, int S, bool FLIP>
-__global__ void __launch_bounds__(TILE_THREADS, KS == 3 ? 3 : 2) dw_tile_kernel(DwArgs a, TilePlan p) {
+__global__ void __launch_bounds__(TILE_THREADS, KS == 3 ? 3 : 2) dw_tile_kernel(const __grid_constant__ DwArgs a, const __grid_constant__ TilePlan p) {
   pdl_wait();
   constexpr int SPAN = (TX - 1) * S + KS, R = (KS + S - 1) / S, U = R * S, KK = KS * KS;
-  constexpr bool WREG = KS <= 5;  // the filter of the thread's two channels in registers
+  constexpr int WROWS = KS == 3 ? 3 : (KS == 5 ? 4 : 0);  // filter rows of the thread's two channels in registers; the fifth row of 5x5 would spill
   extern __shared__ __align__(16) float sm[];
   const int nt = 16 * p.G, t = threadIdx.x, z = threadIdx.y, cp = t & 15, gr = t >> 4;
   const int slabs = (a.c + SLAB - 1) / SLAB;
@@ -110,11 +161,9 @@ __global__ void __launch_bounds__(TILE_THREADS, KS == 3 ? 3 : 2) dw_tile_kernel(
   }
   const bool relu = a.flags & OMT_EPI_RELU;
   __syncthreads();
-  u64 wreg[WREG ? KK : 1];
-  if constexpr (WREG) {
+  u64 wreg[WROWS ? WROWS * KS : 1];
 #pragma unroll
-    for (int k = 0; k < KK; k++) wreg[k] = lds2(wbase + k * SLAB * 4);
-  }
+  for (int k = 0; k < WROWS * KS; k++) wreg[k] = lds2(wbase + k * SLAB * 4);
   float* yrow = a.y.p + (((int64_t)img * a.oh + oy0) * a.ow + ox0) * a.c + ch;
   const int64_t ys = (int64_t)a.ow * a.c;
   const uint32_t lane = ring + (uint32_t)(gr * TX * S * SLAB) * 4 + cp * 8;
@@ -138,7 +187,7 @@ __global__ void __launch_bounds__(TILE_THREADS, KS == 3 ? 3 : 2) dw_tile_kernel(
           if (q < 0 || q >= nrows) continue;
 #pragma unroll
           for (int kx = 0; kx < KS; kx++) {
-            const u64 wv = WREG ? wreg[ky * KS + kx] : lds2(wbase + (ky * KS + kx) * SLAB * 4);
+            const u64 wv = ky < WROWS ? wreg[ky * KS + kx] : lds2(wbase + (ky * KS + kx) * SLAB * 4);
 #pragma unroll
             for (int j = 0; j < TX; j++) fma2(acc[slot][j], in[j * S + kx], wv);
           }
@@ -165,6 +214,9 @@ __global__ void __launch_bounds__(TILE_THREADS, KS == 3 ? 3 : 2) dw_tile_kernel(
       }
     }
   }
+  bool good = true;  // (looked at last: a branch in front of the walk costs it registers)
+  for (int e = threadIdx.y * blockDim.x + threadIdx.x; e < KK * SLAB; e += blockDim.x * blockDim.y) good = good && finite(sm[e]);
+  if (!__syncthreads_and(good)) direct_outputs<KS, S>(a, p, sm);
 }
 
 // Weight gradient: the same walk with a second ring for the rows of gy. A thread keeps the ks * ks tap sums of its two channels
@@ -252,6 +304,7 @@ __global__ void __launch_bounds__(TILE_THREADS, KS == 7 ? 1 : 2) dw_wgrad_tile_k
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   u64* red = reinterpret_cast<u64*>(sm);  // [KS][Z G][16]
   const int lanes = p.Z * p.G, me = z * p.G + gr, tid = z * nt + t;
+  bool good = true;
 #pragma unroll
   for (int ky = 0; ky < KS; ky++) {
     __syncthreads();
@@ -265,9 +318,16 @@ __global__ void __launch_bounds__(TILE_THREADS, KS == 7 ? 1 : 2) dw_wgrad_tile_k
         const float2 v = unpack2(red[(kx * lanes + k) * 16 + c2]);
         s0 += v.x; s1 += v.y;
       }
+      good = good && finite(s0) && finite(s1);
       if (ch < a.c) part[((int64_t)ch * SL + sl) * KK + ky * KS + kx] = s0;
       if (ch + 1 < a.c) part[((int64_t)(ch + 1) * SL + sl) * KK + ky * KS + kx] = s1;
     }
+  }
+  if (__syncthreads_and(good)) return;
+  for (int e = tid; e < SLAB * KK; e += nt * p.Z) {
+    const int ch = ch0 + e % SLAB, tap = e / SLAB;
+    float* o = part + ((int64_t)ch * SL + sl) * KK + tap;
+    if (ch < a.c && !finite(*o)) *o = direct_tap_sum<S>(a, p, sl, SL, ch, tap / KS, tap % KS);
   }
 }
 

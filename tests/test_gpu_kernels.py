@@ -1010,3 +1010,55 @@ def test_pool2_backward_of_channels_last_tensors(capi, shape):
     assert torch.equal(i0.cpu(), i1.cpu())
     want, got = capi.pool2_bwd(dev(gy), i0, (h, w)), capi.pool2_bwd(dev(gy, True), i1, (h, w))
     assert torch.equal(got.cpu(), want.cpu()) and torch.count_nonzero(want) == gy.numel()
+
+
+def depthwise_inside(x, w, gy, s, p):
+    """Output, input gradient and weight gradient of a depthwise convolution in which only pixels inside the image take part."""
+    h, wd, k, oh, ow = x.shape[2], x.shape[3], w.shape[-1], gy.shape[2], gy.shape[3]
+    y, dx, dw = torch.zeros_like(gy), torch.zeros_like(x), torch.zeros_like(w)
+    def span(t, size, out):  # the outputs that see filter row t inside the image, and the pixels they see
+        o0, o1 = max(0, -(-(p - t) // s)), min(out - 1, (size - 1 + p - t) // s)
+        return slice(o0, o1 + 1), slice(o0 * s - p + t, o1 * s - p + t + 1, s), o1 >= o0
+    for ky in range(k):
+        for kx in range(k):
+            (oy, iy, a), (ox, ix, b) = span(ky, h, oh), span(kx, wd, ow)
+            if a and b:
+                xs, gs, wv = x[:, :, iy, ix], gy[:, :, oy, ox], w[:, 0, ky, kx].view(1, -1, 1, 1)
+                y[:, :, oy, ox] += xs * wv
+                dx[:, :, iy, ix] += gs * wv
+                dw[:, 0, ky, kx] = (gs * xs).sum((0, 2, 3))
+    return y, dx, dw
+
+
+@pytest.mark.parametrize("case", [(8, 33, 61, 59, 3, 1, 1), (8, 33, 61, 59, 5, 1, 2), (6, 35, 61, 58, 7, 1, 3), (28, 33, 61, 61, 5, 2, 2), (24, 34, 61, 61, 7, 2, 3), (8, 33, 60, 58, 3, 2, 1), (2, 36, 21, 22, 7, 1, 3), (2, 36, 21, 22, 7, 2, 3)],
+                         ids=lambda t: "x".join(map(str, t)))
+def test_depthwise_leaves_out_pixels_outside_the_image(capi, case):
+    """Infinities and NaNs in filters, pixels and gradients reach the results that use them and no others, with channel counts that are not
+    multiples of four and in 7x7 weight gradients (the other 16-byte kernels multiply zeros in for the pixels outside). The finite results
+    are within (k + 2) 2^-24 of the sum of the k absolute products."""
+    n, c, h, w, ks, s, p = case
+    gen = torch.Generator().manual_seed(sum(case))
+    x, wt = torch.randn(n, c, h, w, generator=gen), torch.randn(c, 1, ks, ks, generator=gen)
+    gy = torch.randn(n, c, (h + 2 * p - ks) // s + 1, (w + 2 * p - ks) // s + 1, generator=gen)
+    eps, inf, nan = 2.0**-24, float("inf"), float("nan")
+
+    def check(got, want, bound):
+        got = got.cpu().double()
+        fin = torch.isfinite(want)
+        assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(got[torch.isinf(want)], want[torch.isinf(want)])
+        assert ((got - want)[fin].abs() <= bound[fin] + 1e-30).all()
+
+    small = [torch.nan_to_num(t, 0, 0, 0).double().abs() for t in (x, wt, gy)]
+    ya, dxa, dwa = depthwise_inside(*small, s, p)
+    wf = wt.clone()
+    wf[0, 0, 0, 0], wf[3, 0, 0, ks - 1], wf[c - 1, 0, ks - 1, ks - 1], wf[2, 0, ks - 1, 0] = inf, nan, -inf, inf
+    y, dx, _ = depthwise_inside(x.double(), wf.double(), gy.double(), s, p)
+    if c % 4:
+        check(capi.dw_fwd(dev(x, True), wf.cuda(), None, s, p, cl=True), y, (ks * ks + 2) * eps * ya)
+        check(capi.dw_dgrad(dev(gy, True), wf.cuda(), (h, w), s, p, cl=True), dx, (ks * ks + 2) * eps * dxa)
+    xf, gf = x.clone(), gy.clone()
+    xf[0, 1, 2, w - 1], xf[n - 1, 2, h - 1, 0], xf[0, 6, h // 2, w // 2], xf[n - 1, c - 1, 0, 0] = inf, nan, -inf, inf
+    gf[0, 4, 0, 0], gf[0, 5, -1, -1], gf[n - 1, c - 1, 1, 1], gf[0, 7, 0, -1] = inf, nan, -inf, -inf
+    _, _, dw = depthwise_inside(xf.double(), wt.double(), gf.double(), s, p)
+    assert torch.isfinite(dw[8:c - 1]).all() and not torch.isfinite(dw[:8]).all()
+    check(capi.dw_wgrad(dev(xf, True), dev(gf, True), ks, s, p), dw, (n * gy.shape[2] * gy.shape[3] + 2) * eps * dwa)
