@@ -893,9 +893,10 @@ struct SplitArgs {
 // window mode: row co, tap = filter row ky, column k' = kx * 4 + c
 __global__ void __launch_bounds__(256) weight_split_kernel(const float* __restrict__ w, float* __restrict__ out, SplitArgs a) {
   pdl_wait();
-  const uint32_t total = (uint32_t)a.co * a.kh * a.cpad, i = blockIdx.x * 256u + threadIdx.x;
+  const int64_t total = (int64_t)a.co * a.kh * a.cpad, i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= total) return;
-  const uint32_t q = i / a.cpad, c = i - q * a.cpad, row = q / a.kh, ty = q - row * a.kh, kx = c >> 2, cc = c & 3;
+  const uint32_t q = i <= 0xffffffffll ? (uint32_t)i / (uint32_t)a.cpad : (uint32_t)(i / a.cpad);
+  const uint32_t c = (uint32_t)(i - (int64_t)q * a.cpad), row = q / a.kh, ty = q - row * a.kh, kx = c >> 2, cc = c & 3;
   const float v = kx < a.ks && cc < a.ci ? __ldg(w + (((int64_t)row * a.ci + cc) * a.ks + ty) * a.ks + kx) : 0.f;
   const float hi = tf32_rna(v);
   out[i] = hi;
@@ -914,7 +915,8 @@ __global__ void __launch_bounds__(256) weight_split_tile_kernel(const float* __r
   __shared__ float sm[SPLIT_FLOATS];
   __shared__ float scale[8];  // of the tile's rows
   const int kk = a.ks * a.ks, rows = DGRAD ? a.ci : a.co, chans = DGRAD ? a.co : a.ci;
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * RB, tid = threadIdx.x;
+  const uint32_t cblocks = a.cpad / 32;  // one grid dimension for both: either extent may be far beyond 65535 (the columns of a matrix product)
+  const int r0 = (int)(blockIdx.x / cblocks) * RB, c0 = (int)(blockIdx.x % cblocks) * 32, tid = threadIdx.x;
   const int run = (DGRAD ? RB : 32) * kk, pitch = run | 1;  // contiguous floats of the original per line; odd pitch: no bank conflicts
   const int lines = DGRAD ? 32 : RB;
   for (int e = tid; e < lines * run; e += 256) {
@@ -925,7 +927,7 @@ __global__ void __launch_bounds__(256) weight_split_tile_kernel(const float* __r
   }
   if (!DGRAD && f.gamma && tid < RB && r0 + tid < rows) {
     scale[tid] = fold_scale(f, r0 + tid);
-    if (blockIdx.x == 0) f.fb[r0 + tid] = fold_bias(f, r0 + tid, scale[tid]);
+    if (c0 == 0) f.fb[r0 + tid] = fold_bias(f, r0 + tid, scale[tid]);
   }
   __syncthreads();
   const int taps = a.kh * a.kw;
@@ -974,7 +976,7 @@ __global__ void __launch_bounds__(256) weight_split_1x1_kernel(const float* __re
 }
 static int split_weights(const float* w, float* out, const SplitArgs& a, const BnFold* fold, cudaStream_t s) {
   const int rows = a.dgrad ? a.ci : a.co, RB = split_rows(a.ks * a.ks);
-  const dim3 grid((unsigned)(a.cpad / 32), (unsigned)cdiv(rows, RB));
+  const unsigned grid = (unsigned)((int64_t)(a.cpad / 32) * cdiv(rows, RB));
   const BnFold f = fold ? *fold : BnFold{};
   if (!a.dgrad && a.ks == 1 && a.ci % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0) {
     launch(weight_split_1x1_kernel, (unsigned)cdiv((int64_t)a.co * (a.cpad / 4), 256), 256, 0, s, w, out, a, f);

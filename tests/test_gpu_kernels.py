@@ -1062,3 +1062,29 @@ def test_depthwise_leaves_out_pixels_outside_the_image(capi, case):
     _, _, dw = depthwise_inside(xf.double(), wt.double(), gf.double(), s, p)
     assert torch.isfinite(dw[8:c - 1]).all() and not torch.isfinite(dw[:8]).all()
     check(capi.dw_wgrad(dev(xf, True), dev(gf, True), ks, s, p), dw, (n * gy.shape[2] * gy.shape[3] + 2) * eps * dwa)
+
+
+@pytest.mark.parametrize("M,K,N,form", [(8, 8, 524_296, "rr"), (3, 40, 600_001, "rr"), (8, 8, 524_289, "shifted"), (8, 100_000, 8, "rr")])
+def test_matrix_products_beyond_a_grid_dimension(capi, M, K, N, form):
+    """More columns than 65535 blocks of the weight re-layout cover, and a long reduction: row-major B (an input gradient) and column-major B
+    that starts 4 bytes past a 16-byte boundary (a forward pass). TOL is the path's own bound; the exact answer in float64."""
+    gen = torch.Generator().manual_seed(N)
+    a, b = torch.randn(M, K, generator=gen).cuda(), torch.randn(K, N, generator=gen).cuda()
+    out = torch.full((M, N), float("nan"), device="cuda")
+    if form == "rr":
+        capi.call("omt_gemm", capi.ptr(a), K, 1, capi.ptr(b), N, 1, None, capi.ptr(out), M, N, K, capi.stream_handle())
+    else:
+        flat = torch.empty(N * K + 1, device="cuda")[1:]
+        flat.view(N, K).copy_(b.t())
+        capi.call("omt_gemm", capi.ptr(a), K, 1, capi.ptr(flat), 1, K, None, capi.ptr(out), M, N, K, capi.stream_handle())
+    assert rel_err(host(out), host(a.double() @ b.double())) <= TOL
+
+
+def test_input_gradient_with_more_channels_than_a_grid_dimension(capi):
+    """A 3x3 layer of 262 148 input channels: its weights are re-laid in blocks of four of them."""
+    ci, co = 262_148, 8
+    gen = torch.Generator().manual_seed(0)
+    gy, wt = torch.randn(1, co, 2, 3, generator=gen), torch.randn(co, ci, 3, 3, generator=gen) / (9 * co) ** 0.5
+    want = torch.nn.functional.conv_transpose2d(gy.double(), wt.double(), padding=1)
+    got = capi.conv_dgrad(dev(gy, True), wt.cuda(), (2, 3), 1, 1, flags=capi.FORCE_TC, cl=True)
+    assert rel_err(host(got), want.numpy()) <= TOL
