@@ -875,3 +875,15 @@ def test_channel_sums_serve_sum_mean_and_global_pooling(omt, shape):
     got = F.adaptive_avg_pool2d(d, 1)
     assert ((got.cpu().double() - x.double().mean((2, 3), True)).abs() <= eps * x.double().abs().mean((2, 3), True)).all()
     assert not omt.FALLBACKS, dict(omt.FALLBACKS)
+
+
+def test_fused_pointwise_long_programs_on_both_sides_of_the_vector_line(omt):
+    """Long programs run four elements per thread from 2^17 elements on: the same bits as from tensors 4 bytes past a boundary, which never do."""
+    fp = torch.ops.omt.fused_pointwise
+    for k in (5, 6, 22):
+        chain = ";".join(["mul,v0,v1,v0"] + [f"add,t{j - 1},{'v0' if j % 2 else 'v1'},#0" if j % 3 else f"tanh,t{j - 1},t0,t0" for j in range(1, k)] + [f"sub,t{k - 1},t2,#0"])
+        for n in (2**17 - 1, 2**17, 2**17 + 3, 200_001):
+            src = [torch.randn(n + 1).to(D), torch.randn(n + 1).to(D)]
+            whole = [t[1:].clone() for t in src]
+            assert torch.equal(fp(f"pw1|2|{chain}|{0.5.hex()}", whole).cpu(), fp(f"pw1|2|{chain}|{0.5.hex()}", [t[1:] for t in src]).cpu()), (k, n)
+    assert not omt.FALLBACKS, dict(omt.FALLBACKS)
