@@ -342,8 +342,9 @@ __global__ void __launch_bounds__(256) maxpool_bwd_nhwc4_fixed_kernel(PoolArgs a
 // Stride 2: one thread takes an even-aligned 2 x 2 block of input pixels. The block meets at most two windows per axis, whose
 // indices and gradients are loaded once and serve all four pixels: 4 window loads per block instead of 9 per-pixel ones
 // (this kernel is bound by the bytes that cross L1, not by HBM). Indices are compared in 32 bits (h * w < 2^31).
+// Five blocks per SM are asked for with 3x3: left alone the compiler takes 56 registers, which is four (256 x 64 x 112 x 112: 338 us, 301 with five).
 template <int KS>
-__global__ void __launch_bounds__(256) maxpool_bwd_nhwc4_s2_block_kernel(PoolArgs a, const int64_t* __restrict__ idx) {
+__global__ void __launch_bounds__(256, KS == 3 ? 5 : 0) maxpool_bwd_nhwc4_s2_block_kernel(PoolArgs a, const int64_t* __restrict__ idx) {
   pdl_wait();
   const int c4 = a.c >> 2, hb = (a.ih + 1) >> 1, wb = (a.iw + 1) >> 1;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
