@@ -224,7 +224,8 @@ class HbmKernels:
         grads = [torch.randn_like(t) for t in params]
         ms_ = [torch.zeros_like(t) for t in params]
         vs_ = [torch.zeros_like(t) for t in params]
-        steps = [torch.zeros((), device="cuda") for _ in params]
+        steps = [torch.ones((), device="cuda") for _ in params]   # (at step 0 both bias corrections are 0 and every quotient is not finite)
+        adam_table = capi.param_table(params, grads, ms_, vs_, steps)
         npar = sum(t.numel() for t in params)
         call = capi.call
         yp, ip = capi.maxpool_fwd(x, 3, 2, 1)   # indices and a gradient for the max-pool backward case
@@ -249,7 +250,7 @@ class HbmKernels:
             "maxpool3x3s2_fwd": (lambda: capi.maxpool_fwd(x, 3, 2, 1), 4 * ne + 12 * (ne // 4)),
             "maxpool3x3s2_bwd": (lambda: capi.maxpool_bwd(gp, ip, (h, w), 3, 2, 1), 4 * ne + 12 * (ne // 4)),
             "sgd_momentum": (lambda: capi.sgd(params, grads, ms_, 0.1, momentum=0.9, weight_decay=1e-4), 20 * npar),
-            "adamw": (lambda: capi.adam(params, grads, ms_, vs_, steps, 1e-3, weight_decay=0.01, decoupled=True), 28 * npar),
+            "adamw": (lambda: call("omt_adam", adam_table, len(params), 1e-3, 0.9, 0.999, 1e-8, 0.01, 1, 0, sh()), 28 * npar),
         }
         self.bytes_resident = 1 << 40
         self.results = {}
