@@ -495,7 +495,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if constexpr (PAIR) cluster_sync_all();  // the other CTA's barriers are initialised before anything here signals them
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
-  pdl_wait();  // everything above touches only this CTA: it overlaps the end of the kernel in front
+  pdl_wait();  // everything above touches only this CTA: it may run while the kernel in front completes and its writes are flushed
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -1397,7 +1397,7 @@ wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
   if constexpr (PAIR) cluster_sync_all();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_acc = *tmem_slot;
-  pdl_wait();  // everything above touches only this CTA: it overlaps the end of the kernel in front
+  pdl_wait();  // everything above touches only this CTA: it may run while the kernel in front completes and its writes are flushed
 
   if (warp == 0) {
     if (lane == 0) {
