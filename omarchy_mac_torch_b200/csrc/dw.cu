@@ -923,6 +923,39 @@ static int launch_rows(const DwArgs& a, const OmtConvGeo* g, float* wt, bool fli
   return check_launch(name);
 }
 
+// Where the tiles of dw_tile.cu take over. A block there computes a slab of 32 channels whether they exist or not, and walks at least ks rows
+// behind one barrier each, 10 to 35 us however little there is to do. So it needs enough channels per slab, and enough pixels to fill the GPU. The
+// lines are where the times of the two kernels cross, warm and with L2 flushed, over 1 to 512 images of 7 to 224 pixels and 2 to 768 channels.
+//
+// Forward and stride-1 input gradient of tensors that the 16-byte kernels cannot take (c % 4 != 0 or unaligned), against one output per thread: 128 x 97 x
+// 56 x 56 3x3 508 -> 206 us, but with 10 channels 56 -> 65, and 128 x 33 x 7 x 7 8 -> 12. The input gradient of one output per thread is slower than its
+// forward pass, so its lines are lower; forward 3x3 stride 2 reads so little per output that tiles hardly ever pay. (The 16-byte kernels
+// themselves are faster than tiles: 128 x 96 x 56 x 56 5x5 118 us against 136, 3x3 67 against 85.)
+static bool tile_conv_pays(const DwArgs& a, bool flip) {
+  struct Line { int channels; int64_t outputs; };  // channels per slab, outputs in all; for 3x3, 5x5, 7x7
+  static constexpr Line grad1[3] = {{6, 300000}, {5, 200000}, {5, 200000}}, fwd1[3] = {{14, 800000}, {8, 400000}, {9, 500000}},
+                        fwd2[3] = {{17, 3000000}, {17, 1000000}, {14, 500000}};
+  const Line l = (flip ? grad1 : (a.stride == 2 ? fwd2 : fwd1))[a.ks / 2 - 1];
+  return a.c >= l.channels * cdiv(a.c, 32) && (int64_t)a.n * a.c * a.oh * a.ow >= l.outputs;
+}
+// Weight gradient. Against the 16-byte kernels: 3x3 stride 1 up to 2^16 output pixels (128 x 36 x 14 x 14 14.7 -> 10.6 us, but 128 x 36 x 56 x 56 39 ->
+// 58, 96 channels 76 -> 81), 5x5 stride 2 always (64 x 96 x 112 x 112 189 -> 131), images at most eight pixels wide (128 x 48 x 7 x 7 19.5 -> 13.3);
+// 5x5 stride 1 and 3x3 stride 2 else never (32 x 240 x 14 x 14 23.6 -> 26.7, 32 x 72 x 56 x 56 27.5 -> 30.0). Against a thread per channel (at least 32
+// channels): always (128 x 97 x 56 x 56 3x3 581 -> 245), but for a few pixels at stride 2. Against a block per channel and group of images (below 32
+// channels): that kernel's time is the chain of its 256-pixel steps, longer where its blocks outnumber the SMs; a tile's is the pixels of all images (2 x 5 x
+// 224 x 224 5x5 207 -> 37, but 32 x 5 x 112 x 112 74 -> 129). Below 7x7 a small image costs a tile as much as 256 pixels.
+static bool tile_wgrad_pays(const DwArgs& a, bool vec) {
+  const int64_t ohw = (int64_t)a.oh * a.ow, pixels = a.n * ohw;
+  if (vec && a.ks < 7) return a.ow <= 8 || (a.ks == 3 && a.stride == 1 && pixels < 1 << 16) || (a.ks == 5 && a.stride == 2);
+  if (a.c >= 32) return a.ks == 7 || a.stride == 1 || pixels >= 512;
+  struct Line { double blocks_per_sm, base, per_4096_pixels; };
+  static constexpr Line small[2] = {{1.5, 3, 1.5}, {0.5, 20, 4}}, seven[2] = {{1.5, 4, 0.7}, {0.5, 10, 4}}, seven_vec = {0.75, 2, 0.7};  // by stride
+  const Line l = a.ks < 7 ? small[a.stride - 1] : (vec ? seven_vec : seven[a.stride - 1]);
+  const int64_t slices = std::min<int64_t>(a.n, cdiv(4 * sm_count(), a.c));
+  const double chain = (double)(cdiv(a.n, slices) * cdiv(ohw, 256)) * std::max(1.0, (double)(a.c * slices) / (l.blocks_per_sm * sm_count()));
+  return chain >= l.base + l.per_4096_pixels * (double)(a.n * std::max<int64_t>(ohw, a.ks < 7 ? 256 : 0)) / 4096;
+}
+
 }  // namespace omt
 
 using namespace omt;
@@ -938,10 +971,7 @@ int omt_dw_fwd(const OmtConvGeo* g, const OmtAct* x, const float* w, const float
   bool xn = is_nhwc(x, g->ci, g->ih, g->iw), yn = is_nhwc(y, g->co, g->oh, g->ow);
   int64_t total = (int64_t)g->n * g->co * g->oh * g->ow;
   const bool vec = g->ci % 4 == 0 && aligned16(x->p) && aligned16(y->p) && (!bias || aligned16(bias));
-  // tiles where the 16-byte kernels cannot go (64 x 97 x 56 x 50 5x5: forward 461 -> 170 us, input gradient 946 -> 172; 64 x 130 x 40 x 40
-  // 7x7: 738 -> 141 and 1249 -> 141); where they can, a thread's private ring without barriers is faster (128 x 96 x 56 x 56: 5x5 118
-  // against 136, 3x3 67 against 85)
-  if (xn && yn && !vec && dw_tile_ok(a)) return dw_tile_conv(a, false, st(stream));
+  if (xn && yn && !vec && dw_tile_ok(a) && tile_conv_pays(a, false)) return dw_tile_conv(a, false, st(stream));
   if (xn && yn && vec) {
     if (rows_ok(g)) {
       Scratch sc;
@@ -969,9 +999,10 @@ int omt_dw_dgrad(const OmtConvGeo* g, const OmtAct* gy, const float* w, const Om
     // stride 1: the forward kernel over gy with mirrored taps, as below
     DwArgs f = a;
     f.ih = g->oh; f.iw = g->ow; f.oh = g->ih; f.ow = g->iw; f.pad = g->ks - 1 - g->pad;
-    if (dw_tile_ok(f)) return dw_tile_conv(f, true, st(stream));
+    if (dw_tile_ok(f) && tile_conv_pays(f, true)) return dw_tile_conv(f, true, st(stream));
   }
-  if (nhwc && !vec && g->stride == 2 && rows_ok(g)) {
+  // (one channel per thread on few pixels: the re-laid filter is a launch more than the general kernel needs, 10 us against 8 up to about these sizes)
+  if (nhwc && !vec && g->stride == 2 && rows_ok(g) && total >= (g->ks == 3 ? 400000 : (g->ks == 5 ? 150000 : 80000))) {
     Scratch sc;
     const int kk = g->ks * g->ks;
     r = sc.get(nullptr, 0, (size_t)g->ci * kk * sizeof(float), stream);
@@ -1018,24 +1049,17 @@ int omt_dw_wgrad(const OmtConvGeo* g, const OmtAct* x, const OmtAct* gy, float* 
   DwArgs a = mk(g, x, gy, nullptr, nullptr, 0);
   cudaStream_t s = st(stream);
   const int c = g->ci, kk = g->ks * g->ks;
-  if (is_nhwc(x, c, g->ih, g->iw) && is_nhwc(gy, c, g->oh, g->ow) && dw_tile_ok(a)) {
-    const bool vec = c % 4 == 0 && aligned16(x->p) && aligned16(gy->p);
-    // tiles, but for the two cases where the 16-byte kernels keep up: 5x5 stride 1 (32 x 240 x 14 x 14 23.6 us against 26.7) and 3x3
-    // stride 2 (32 x 72 x 56 x 56 27.5 against 30.0). Else (old against tiles): 7x7 64 x 96 x 56 x 56 1564 and 122 us; 5x5 stride 2 64 x 96 x
-    // 112 x 112 189 and 131; 3x3 128 x 96 x 56 x 56 91 and 86, 128 x 48 x 7 x 7 19.5 and 13.3; no multiple of four channels, 64 x 97 x 56 x 50
-    // 5x5, 452 and 212
-    if (!vec || g->ks == 7 || (g->ks == 5) == (g->stride == 2) || g->ow <= 8) return dw_tile_wgrad(a, vec, scale, dw, stream);
-  }
+  const bool vec = c % 4 == 0 && aligned16(x->p) && aligned16(gy->p);
+  if (is_nhwc(x, c, g->ih, g->iw) && is_nhwc(gy, c, g->oh, g->ow) && dw_tile_ok(a) && tile_wgrad_pays(a, vec)) return dw_tile_wgrad(a, vec, scale, dw, stream);
   const bool nhwc = is_nhwc(x, c, g->ih, g->iw) && is_nhwc(gy, c, g->oh, g->ow) && c >= 32;
   const bool reg = g->ks == 3 || g->ks == 5 || g->ks == 7;
-  if (is_nhwc(x, c, g->ih, g->iw) && is_nhwc(gy, c, g->oh, g->ow) && c % 4 == 0 && aligned16(x->p) && aligned16(gy->p) &&
-      ((g->ks == 5 && g->stride == 1) || (g->ks == 3 && g->stride == 2))) {
+  if (is_nhwc(x, c, g->ih, g->iw) && is_nhwc(gy, c, g->oh, g->ow) && vec && ((g->ks == 5 && g->stride == 1) || (g->ks == 3 && g->stride <= 2))) {
     float* part = nullptr;
     int S = 1;
     Scratch sc;
     if (g->stride == 1) {
-      // rolling strips; 2 channels per thread (25 tap sums per channel)
-      const int CH = 2, TX = 4;
+      // rolling strips; 4 channels per thread for 3x3, 2 for 5x5 (25 tap sums per channel)
+      const int CH = g->ks == 3 ? 4 : 2, TX = 4;
       const int cqn = c / CH;
       const int CL = std::min(cqn, 32), PL = ROLL_THREADS / CL;
       const int gx = (int)cdiv(cqn, CL);
@@ -1049,7 +1073,8 @@ int omt_dw_wgrad(const OmtConvGeo* g, const OmtAct* x, const OmtAct* gy, float* 
       if (r) return r;
       part = (float*)sc.p;
       dim3 grid(gx, S);
-      launch_wgrad_roll<5, 1, 4, 2>(a, grid, S, CL, rows, segs, part, s);
+      if (g->ks == 3) launch_wgrad_roll<3, 1, 4, 4>(a, grid, S, CL, rows, segs, part, s);
+      else launch_wgrad_roll<5, 1, 4, 2>(a, grid, S, CL, rows, segs, part, s);
     } else {  // stride 2: a group of four output pixels per trip (measured 0.77 of the copy bandwidth against 0.61 for strips)
       const int c4 = c / 4;
       const int CL = std::min(c4, 32), PL = 256 / CL;

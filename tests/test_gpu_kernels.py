@@ -1030,7 +1030,7 @@ def depthwise_inside(x, w, gy, s, p):
     return y, dx, dw
 
 
-@pytest.mark.parametrize("case", [(8, 33, 61, 59, 3, 1, 1), (8, 33, 61, 59, 5, 1, 2), (6, 35, 61, 58, 7, 1, 3), (28, 33, 61, 61, 5, 2, 2), (24, 34, 61, 61, 7, 2, 3), (8, 33, 60, 58, 3, 2, 1), (2, 36, 21, 22, 7, 1, 3), (2, 36, 21, 22, 7, 2, 3)],
+@pytest.mark.parametrize("case", [(8, 33, 61, 59, 3, 1, 1), (8, 33, 61, 59, 5, 1, 2), (6, 35, 61, 58, 7, 1, 3), (34, 33, 61, 61, 5, 2, 2), (24, 34, 61, 61, 7, 2, 3), (8, 33, 60, 58, 3, 2, 1), (2, 36, 21, 22, 7, 1, 3), (2, 36, 21, 22, 7, 2, 3)],
                          ids=lambda t: "x".join(map(str, t)))
 def test_depthwise_leaves_out_pixels_outside_the_image(capi, case):
     """Infinities and NaNs in filters, pixels and gradients reach the results that use them and no others, with channel counts that are not
@@ -1088,3 +1088,40 @@ def test_input_gradient_with_more_channels_than_a_grid_dimension(capi):
     want = torch.nn.functional.conv_transpose2d(gy.double(), wt.double(), padding=1)
     got = capi.conv_dgrad(dev(gy, True), wt.cuda(), (2, 3), 1, 1, flags=capi.FORCE_TC, cl=True)
     assert rel_err(host(got), want.numpy()) <= TOL
+
+
+DW_LINES = [  # n, c, h, w, ks, stride, pad, tensors' offset in floats, the kernels that serve it among those looked at
+    (16, 5, 60, 61, 3, 1, 1, 0, []), (128, 33, 7, 7, 3, 1, 1, 0, ["dw_wgrad_tile"]), (8, 34, 62, 61, 3, 1, 1, 0, ["dw_dgrad_tile", "dw_fwd_tile", "dw_wgrad_tile"]),
+    (40, 10, 41, 39, 3, 1, 1, 0, ["dw_dgrad_tile"]), (28, 33, 61, 58, 3, 2, 1, 0, ["dw_dgrad_s2_nhwc", "dw_wgrad_tile"]), (4, 97, 203, 201, 3, 2, 1, 0, ["dw_dgrad_s2_nhwc", "dw_fwd_tile", "dw_wgrad_tile"]),
+    (9, 31, 43, 47, 5, 1, 2, 0, ["dw_dgrad_tile", "dw_fwd_tile", "dw_wgrad_tile"]), (36, 35, 61, 59, 5, 2, 2, 0, ["dw_dgrad_s2_nhwc", "dw_fwd_tile", "dw_wgrad_tile"]), (4, 6, 37, 35, 5, 2, 2, 0, []),
+    (7, 45, 44, 43, 7, 1, 3, 0, ["dw_dgrad_tile", "dw_fwd_tile", "dw_wgrad_tile"]), (24, 43, 53, 51, 7, 2, 3, 0, ["dw_dgrad_s2_nhwc", "dw_fwd_tile", "dw_wgrad_tile"]), (5, 3, 19, 21, 7, 2, 3, 0, []),
+    (2, 5, 200, 199, 3, 1, 1, 0, ["dw_wgrad_tile"]), (3, 7, 150, 181, 5, 1, 2, 0, ["dw_dgrad_tile", "dw_wgrad_tile"]), (32, 6, 70, 66, 3, 1, 1, 0, ["dw_dgrad_tile"]),
+    (32, 8, 112, 111, 3, 1, 1, 0, ["dw_wgrad_strips_nhwc"]), (32, 36, 57, 56, 3, 1, 1, 0, ["dw_wgrad_strips_nhwc"]), (21, 36, 57, 56, 3, 1, 1, 0, ["dw_wgrad_strips_nhwc"]), (20, 36, 57, 56, 3, 1, 1, 0, ["dw_wgrad_tile"]),
+    (32, 16, 14, 14, 3, 1, 1, 0, ["dw_wgrad_tile"]), (1100, 4, 8, 8, 3, 1, 1, 0, ["dw_wgrad_tile"]), (16, 24, 31, 30, 3, 2, 1, 0, ["dw_wgrad_nhwc4"]), (16, 24, 31, 30, 5, 1, 2, 0, ["dw_wgrad_strips_nhwc"]),
+    (16, 24, 31, 30, 5, 2, 2, 0, ["dw_wgrad_tile"]), (16, 8, 30, 30, 7, 2, 3, 0, []), (64, 8, 56, 56, 7, 2, 3, 0, ["dw_wgrad_tile"]), (12, 36, 50, 47, 3, 1, 1, 1, ["dw_dgrad_tile", "dw_fwd_tile", "dw_wgrad_tile"]),
+]
+
+
+@pytest.mark.parametrize("case", DW_LINES, ids=lambda t: "x".join(map(str, t[:8])))
+def test_depthwise_kernels_on_both_sides_of_their_lines(capi, case):
+    """Which of the depthwise kernels of channels-last tensors runs, at real sizes with few and many channels, and its results against float64: a sum of
+    k products in float32 is within (k + 2) 2^-24 of the sum of their absolute values."""
+    n, c, h, w, ks, s, p, shift, names = case
+    gen = torch.Generator().manual_seed(sum(case[:8]))
+
+    def place(*shape):
+        m, ch, hh, ww = shape
+        flat = torch.empty(m * ch * hh * ww + 4, device="cuda")[shift:shift + m * ch * hh * ww]
+        flat.copy_(torch.randn(flat.shape, generator=gen))
+        return flat.view(m, hh, ww, ch).permute(0, 3, 1, 2)
+    x, gy = place(n, c, h, w), place(n, c, (h + 2 * p - ks) // s + 1, (w + 2 * p - ks) // s + 1)
+    wt = torch.randn(c, 1, ks, ks, generator=gen).cuda()
+    capi.kernel_counts(reset=True)
+    got = capi.dw_fwd(x, wt, None, s, p, cl=True), capi.dw_dgrad(gy, wt, (h, w), s, p, cl=True), capi.dw_wgrad(x, gy, ks, s, p)
+    ran = capi.kernel_counts()
+    seen = ["dw_dgrad_tile", "dw_fwd_tile", "dw_wgrad_tile", "dw_wgrad_strips_nhwc", "dw_wgrad_nhwc4"] + (["dw_dgrad_s2_nhwc"] if c % 4 else [])
+    assert sorted(k for k in seen if ran.get(k)) == sorted(names), ran
+    want = depthwise_inside(x.double(), wt.double(), gy.double(), s, p)
+    size = depthwise_inside(x.double().abs(), wt.double().abs(), gy.double().abs(), s, p)
+    for v, ref, bound, k in zip(got, want, size, (ks * ks, ks * ks, gy.numel() // c)):
+        assert ((v.double() - ref).abs() <= (k + 2) * 2.0**-24 * bound + 1e-30).all()
