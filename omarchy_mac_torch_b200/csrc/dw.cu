@@ -307,10 +307,9 @@ __global__ void __launch_bounds__(256) dw_dgrad_nhwc4_kernel(DwArgs a, const flo
 // A work item is a group of TX = 4 consecutive pixels of one output row: per filter row its (TX-1)*stride + KS input pixels
 // and the 4 gy pixels are loaded together (enough loads in flight to cover DRAM latency at one block per SM), then
 // every tap takes its 4 products from registers.
-template <int KS, int STRIDE>
 __global__ void __launch_bounds__(256) dw_wgrad_nhwc4_kernel(DwArgs a, int S, int CL, float* __restrict__ part) {
   pdl_wait();
-  constexpr int TX = 4, SPAN = (TX - 1) * STRIDE + KS;
+  constexpr int KS = 3, STRIDE = 2, TX = 4, SPAN = (TX - 1) * STRIDE + KS;
   extern __shared__ float4 red4[];  // [PL][CL]
   const int PL = blockDim.x / CL;
   const int cl = threadIdx.x % CL, pl = threadIdx.x / CL;
@@ -719,10 +718,10 @@ __global__ void __launch_bounds__(256) dw_dgrad_s2_kernel(DwArgs a, const float*
 // Weight gradient, rolling: a (channel group, pixel lane) thread walks strips of TX columns x seg_rows output rows; an input row
 // is loaded once and meets the R gy rows it overlaps (kept in registers), every tap's sum stays in registers for the
 // whole walk. Pixel lanes are summed through shared memory in a fixed order, slices (blockIdx.y) by dw_wgrad_fin_kernel.
-template <int KS, int S, int TX, int CH>
+template <int KS, int CH>
 __global__ void __launch_bounds__(ROLL_THREADS) dw_wgrad_roll_kernel(DwArgs a, int SL, int CL, int seg_rows, int segs, float* __restrict__ part) {
   pdl_wait();
-  constexpr int SPAN = (TX - 1) * S + KS, R = (KS + S - 1) / S, U = R * S;
+  constexpr int TX = 4, SPAN = TX - 1 + KS;  // stride 1
   extern __shared__ __align__(16) uint8_t ring_raw[];  // the row ring; after the walk its start is reused as [PL][CL] vectors of CH floats
   const int PL = blockDim.x / CL;
   const int cl = threadIdx.x % CL, pl = threadIdx.x / CL;
@@ -742,16 +741,16 @@ __global__ void __launch_bounds__(ROLL_THREADS) dw_wgrad_roll_kernel(DwArgs a, i
       const uint32_t xg = it % gx, r_ = it / gx;
       const int seg = (int)(r_ % (uint32_t)segs), img = (int)(r_ / (uint32_t)segs);
       const int ox0 = (int)xg * TX, oy_begin = seg * seg_rows, nrows = min(seg_rows, a.oh - oy_begin);
-      const int sy0 = oy_begin * S - a.pad, x0 = ox0 * S - a.pad;
-      const int n_in = (nrows - 1) * S + KS;
+      const int sy0 = oy_begin - a.pad, x0 = ox0 - a.pad;
+      const int n_in = nrows - 1 + KS;
       const float* xbase = a.x.p + (((int64_t)img * a.ih + sy0) * a.iw + x0) * a.c + ch;
       const float* gbase = a.y.p + (((int64_t)img * a.oh + oy_begin) * a.ow + ox0) * a.c + ch;
       const bool gfull = ox0 + TX <= a.ow;
-      Vec<CH> g[R][TX];
+      Vec<CH> g[KS][TX];
       auto row_valid = [&](int r) { return r < n_in && sy0 + r >= 0 && sy0 + r < a.ih; };
 #pragma unroll
       for (int d = 0; d < ROLL_DEPTH; d++) ring.request(d, row_valid(d), xbase + d * rs, safe, x0, a.iw, a.c);
-      if constexpr (S == 1 && KS >= 5) {  // one input row per trip, g[ky] = the gy row this input row is filter row ky of (see dw_roll_kernel)
+      if constexpr (KS >= 5) {  // one input row per trip, g[ky] = the gy row this input row is filter row ky of (see dw_roll_kernel)
 #pragma unroll 1
         for (int r = 0; r < n_in; r++) {
 #pragma unroll
@@ -786,16 +785,12 @@ __global__ void __launch_bounds__(ROLL_THREADS) dw_wgrad_roll_kernel(DwArgs a, i
         }
         continue;
       }
-      for (int base = 0; base < n_in; base += U) {
-        const int qb = base / S;
+      for (int base = 0; base < n_in; base += KS) {
 #pragma unroll
-        for (int u = 0; u < U; u++) {
+        for (int u = 0; u < KS; u++) {
           const int r = base + u;
           if (r >= n_in) break;
-          if (u % S == 0) {  // the first input row of output row q: its gy pixels enter the ring
-            const int dq = u / S, slot = dq % R, q = qb + dq;
-            if (q < nrows) load_span<CH, TX>(g[slot], gbase + (int64_t)q * a.ow * a.c, ox0, a.ow, a.c, gfull);
-          }
+          if (r < nrows) load_span<CH, TX>(g[u], gbase + (int64_t)r * a.ow * a.c, ox0, a.ow, a.c, gfull);  // the first input row of output row r: its gy pixels enter the ring
           ring.wait_oldest();
           const bool have = row_valid(r);
           Vec<CH> in[SPAN];
@@ -804,14 +799,12 @@ __global__ void __launch_bounds__(ROLL_THREADS) dw_wgrad_roll_kernel(DwArgs a, i
           if (!have) continue;
 #pragma unroll
           for (int ky = 0; ky < KS; ky++) {
-            if (pos_mod(u - ky, S) != 0) continue;
-            const int dq = floor_div(u - ky, S), slot = pos_mod(dq, R);
-            const int q = qb + dq;
+            const int slot = pos_mod(u - ky, KS), q = r - ky;
             if (q < 0 || q >= nrows) continue;
 #pragma unroll
             for (int kx = 0; kx < KS; kx++)
 #pragma unroll
-              for (int j = 0; j < TX; j++) fmav<CH>(acc[ky * KS + kx], g[slot][j], in[j * S + kx]);
+              for (int j = 0; j < TX; j++) fmav<CH>(acc[ky * KS + kx], g[slot][j], in[j + kx]);
           }
         }
       }
@@ -889,11 +882,11 @@ static void launch_roll(const DwArgs& a, const float* wt, cudaStream_t s) {
   allow_shared_memory<dw_roll_kernel<KS, S, FLIP, TX, CH, WREG>>(smem);
   launch(dw_roll_kernel<KS, S, FLIP, TX, CH, WREG>, (unsigned)cdiv(per_seg * segs, ROLL_THREADS), ROLL_THREADS, smem, s, a, wt, rows, segs);
 }
-template <int KS, int S, int TX, int CH>
+template <int KS, int CH>
 static void launch_wgrad_roll(const DwArgs& a, dim3 grid, int SL, int CL, int rows, int segs, float* part, cudaStream_t s) {
-  constexpr size_t smem = ring_bytes<CH, (TX - 1) * S + KS>();
-  allow_shared_memory<dw_wgrad_roll_kernel<KS, S, TX, CH>>(smem);
-  launch(dw_wgrad_roll_kernel<KS, S, TX, CH>, grid, ROLL_THREADS, smem, s, a, SL, CL, rows, segs, part);
+  constexpr size_t smem = ring_bytes<CH, 3 + KS>();
+  allow_shared_memory<dw_wgrad_roll_kernel<KS, CH>>(smem);
+  launch(dw_wgrad_roll_kernel<KS, CH>, grid, ROLL_THREADS, smem, s, a, SL, CL, rows, segs, part);
 }
 // Which kernel serves which case (measured on 128 x 96 x 56 x 56 and 64 x 96 x 112 x 112 -> 56 x 56, fraction of the copy
 // bandwidth): stride 1, 3x3 and 5x5: the rolling kernel (3x3: 0.75 against 0.66); stride 2 and 7x7: one output row per thread
@@ -1073,8 +1066,8 @@ int omt_dw_wgrad(const OmtConvGeo* g, const OmtAct* x, const OmtAct* gy, float* 
       if (r) return r;
       part = (float*)sc.p;
       dim3 grid(gx, S);
-      if (g->ks == 3) launch_wgrad_roll<3, 1, 4, 4>(a, grid, S, CL, rows, segs, part, s);
-      else launch_wgrad_roll<5, 1, 4, 2>(a, grid, S, CL, rows, segs, part, s);
+      if (g->ks == 3) launch_wgrad_roll<3, 4>(a, grid, S, CL, rows, segs, part, s);
+      else launch_wgrad_roll<5, 2>(a, grid, S, CL, rows, segs, part, s);
     } else {  // stride 2: a group of four output pixels per trip (measured 0.77 of the copy bandwidth against 0.61 for strips)
       const int c4 = c / 4;
       const int CL = std::min(c4, 32), PL = 256 / CL;
@@ -1086,7 +1079,7 @@ int omt_dw_wgrad(const OmtConvGeo* g, const OmtAct* x, const OmtAct* gy, float* 
       part = (float*)sc.p;
       dim3 grid(gx, S);
       const size_t smem = (size_t)PL * CL * sizeof(float4);
-      launch(dw_wgrad_nhwc4_kernel<3, 2>, grid, 256, smem, s, a, S, CL, part);
+      launch(dw_wgrad_nhwc4_kernel, grid, 256, smem, s, a, S, CL, part);
     }
     r = check_launch(g->stride == 1 ? "dw_wgrad_strips_nhwc" : "dw_wgrad_nhwc4");
     if (r) return r;
