@@ -482,7 +482,7 @@ class Train:
             kt = self.core.kernel_times(True)
         finally:
             self.core.debug_time_kernels(False)
-        helpers = ("conv_tc_weight_split", "conv_tc_stage_window", "conv_tc_splitk_epilogue", "wgrad_tc_reduce")
+        helpers = ("conv_tc_weight_split", "conv_tc_weight_split_tiles", "conv_tc_stage_window", "conv_tc_splitk_epilogue", "wgrad_tc_reduce")
         gemm_ms = sum(v for k, v in kt.items() if k.startswith(("conv_tc_", "wgrad_tc_")) and k not in helpers)
         helper_ms = sum(v for k, v in kt.items() if k in helpers)
         sustained = peaks.get("bf16_tflops_sustained") or peaks["bf16_tflops"]

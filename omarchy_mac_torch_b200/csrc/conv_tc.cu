@@ -890,23 +890,40 @@ struct SplitArgs {
   int co, ci, ks, kh, kw, cpad, dgrad, ky0, kx0, step;
   int window;  // forward, window mode: tap = filter row ky, column k' = kx*4 + c
 };
-// window mode: row co, tap = filter row ky, column k' = kx * 4 + c
-__global__ void __launch_bounds__(256) weight_split_kernel(const float* __restrict__ w, float* __restrict__ out, SplitArgs a) {
+// One thread per element of a plane: window mode, the few taps of a stride phase, small filters. With `f` an eval BatchNorm of the output is
+// folded in on the way (BnFold; not in window mode).
+__global__ void __launch_bounds__(256) weight_split_kernel(const float* __restrict__ w, float* __restrict__ out, SplitArgs a, const BnFold f) {
   pdl_wait();
-  const int64_t total = (int64_t)a.co * a.kh * a.cpad, i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  const int rows = a.dgrad ? a.ci : a.co, chans = a.window ? a.cpad : (a.dgrad ? a.co : a.ci), kk = a.kh * a.kw;
+  const int64_t total = (int64_t)rows * kk * a.cpad, i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= total) return;
   const uint32_t q = i <= 0xffffffffll ? (uint32_t)i / (uint32_t)a.cpad : (uint32_t)(i / a.cpad);
-  const uint32_t c = (uint32_t)(i - (int64_t)q * a.cpad), row = q / a.kh, ty = q - row * a.kh, kx = c >> 2, cc = c & 3;
-  const float v = kx < a.ks && cc < a.ci ? __ldg(w + (((int64_t)row * a.ci + cc) * a.ks + ty) * a.ks + kx) : 0.f;
+  const int c = (int)(i - (int64_t)q * a.cpad), row = (int)(q / (uint32_t)kk), tap = (int)(q - (uint32_t)row * kk);
+  float v = 0.f;
+  if (c < chans) {
+    const int ty = tap / a.kw, tx = tap - ty * a.kw;
+    if (a.window) {
+      const int kx = c >> 2, cc = c & 3;
+      if (kx < a.ks && cc < a.ci) v = __ldg(w + (((int64_t)row * a.ci + cc) * a.ks + ty) * a.ks + kx);
+    } else if (a.dgrad) {
+      v = __ldg(w + (((int64_t)c * a.ci + row) * a.ks + a.ky0 + a.step * (a.kh - 1 - ty)) * a.ks + a.kx0 + a.step * (a.kw - 1 - tx));
+    } else {
+      v = __ldg(w + (((int64_t)row * a.ci + c) * a.ks + ty) * a.ks + tx);
+    }
+  }
+  if (f.gamma) {
+    const float scale = fold_scale(f, row);
+    v = __fmul_rn(v, scale);
+    if (c == 0 && tap == 0) f.fb[row] = fold_bias(f, row, scale);
+  }
   const float hi = tf32_rna(v);
   out[i] = hi;
   out[total + i] = tf32_rna(v - hi);
 }
 
-// The same re-layout, everything but window mode, as tiles of 32 channels x RB rows x all taps through shared memory: both the reads
-// (runs of channels x taps, or in dgrad rows x taps, of the original) and the writes (32 channels of one tap) are contiguous. An
-// eval BatchNorm of the output is folded in on the way (BnFold): an eval pass of ResNet-50, batch 32, 3148 -> 3021 us against
-// folding into a copy of the weights first; on its own the tiling left the training steps where they were.
+// The same re-layout of a whole filter as tiles of 32 channels x RB rows x all taps through shared memory: both the reads (runs of channels x
+// taps, or in dgrad rows x taps, of the original) and the writes (32 channels of one tap) are contiguous. A block reads all taps of its rows, so
+// it is no kernel for a stride phase.
 constexpr int SPLIT_FLOATS = 4096;
 constexpr int split_rows(int kk) { return kk == 1 ? 8 : (kk <= 9 ? 4 : (kk <= 49 ? 2 : 1)); }  // many small blocks; 32 * (split_rows(kk) * kk | 1) <= SPLIT_FLOATS up to 11 x 11
 template <bool DGRAD>
@@ -974,16 +991,25 @@ __global__ void __launch_bounds__(256) weight_split_1x1_kernel(const float* __re
   *reinterpret_cast<float4*>(o) = make_float4(hi[0], hi[1], hi[2], hi[3]);
   *reinterpret_cast<float4*>(o + (int64_t)a.co * a.cpad) = make_float4(lo[0], lo[1], lo[2], lo[3]);
 }
+// Tiles where their contiguous reads outweigh two passes through a block (element by element -> tiles, warm): a whole filter of 3x3 and more
+// with 2^16 rows x channels and more (512 x 512 3x3 16.2 -> 13.4 us, 256 x 256 5.2 -> 5.0, but 64 x 64 1.7 -> 2.9), and the transposition of
+// a 1x1 filter below 2^18 (256 x 256 2.2 -> 1.8, but 2048 x 2048 28.6 -> 32.6). A stride phase of a 512 x 512 3x3 filter: 3.3 -> 7.2 us with one tap, 8.4 ->
+// 9.8 with four. These ratios hold with L2 flushed.
 static int split_weights(const float* w, float* out, const SplitArgs& a, const BnFold* fold, cudaStream_t s) {
-  const int rows = a.dgrad ? a.ci : a.co, RB = split_rows(a.ks * a.ks);
-  const unsigned grid = (unsigned)((int64_t)(a.cpad / 32) * cdiv(rows, RB));
+  const int rows = a.dgrad ? a.ci : a.co, chans = a.dgrad ? a.co : a.ci, RB = split_rows(a.ks * a.ks);
   const BnFold f = fold ? *fold : BnFold{};
-  if (!a.dgrad && a.ks == 1 && a.ci % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0) {
+  if (!a.window && !a.dgrad && a.ks == 1 && a.ci % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0) {
     launch(weight_split_1x1_kernel, (unsigned)cdiv((int64_t)a.co * (a.cpad / 4), 256), 256, 0, s, w, out, a, f);
     return check_launch("conv_tc_weight_split");
   }
-  if (a.dgrad) launch(weight_split_tile_kernel<true>, grid, 256, 0, s, w, out, a, RB, f);
-  else launch(weight_split_tile_kernel<false>, grid, 256, 0, s, w, out, a, RB, f);
+  const int64_t elements = (int64_t)rows * chans;
+  if (!a.window && a.kh == a.ks && a.kw == a.ks && (a.ks == 1 ? a.dgrad && elements < 1 << 18 : elements >= 1 << 16)) {
+    const unsigned grid = (unsigned)((int64_t)(a.cpad / 32) * cdiv(rows, RB));
+    if (a.dgrad) launch(weight_split_tile_kernel<true>, grid, 256, 0, s, w, out, a, RB, f);
+    else launch(weight_split_tile_kernel<false>, grid, 256, 0, s, w, out, a, RB, f);
+    return check_launch("conv_tc_weight_split_tiles");
+  }
+  launch(weight_split_kernel, (unsigned)cdiv((int64_t)rows * a.kh * a.kw * a.cpad, 256), 256, 0, s, w, out, a, f);
   return check_launch("conv_tc_weight_split");
 }
 
@@ -1770,9 +1796,7 @@ int run_window_fwd(const OmtConvGeo* g, const OmtAct* x, const float* w, const f
   a.cblocks = wp.kb; a.flags = flags; a.stats = stats;
   a.win_w = wp.win_w; a.win_h = wp.win_h; a.tiles_x = wp.tiles_x; a.tiles_y = wp.tiles_y;
   SplitArgs sp{g->co, g->ci, g->ks, g->ks, 1, wp.kb * BKF, 0, 0, 0, 1, 1};
-  const int64_t wtotal = (int64_t)g->co * g->ks * wp.kb * BKF;
-  launch(weight_split_kernel, (unsigned)cdiv(wtotal, 256), 256, 0, s, w, wsplit, sp);
-  r = check_launch("conv_tc_weight_split");
+  r = split_weights(w, wsplit, sp, nullptr, s);
   if (r) return r;
   const int bn = g->co <= 64 ? 64 : (g->co <= 128 ? 128 : 256);
   switch (bn) {
