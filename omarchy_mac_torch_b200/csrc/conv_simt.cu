@@ -335,7 +335,8 @@ struct WgradCl : Wgrad {
 // outputs over very many pixels (16 x 32 outputs, eight groups), which a 128 x 64 tile computes almost entirely as padding: 252 us
 // for 16 x 27 outputs over 401 408 pixels, 7 % of a MobileNetV3 step. With the channels-last loaders the three passes of a
 // 90 -> 50 channel 3x3 stride-2 layer (13 x 57 x 43) go from 217 to 151 us, that step from 3783 to 3592.
-// (0: no minimum number of blocks. A minimum of one lets the compiler spend registers freely: 155 against 126 for the 128 x 128 weight gradient,
+// (0: no minimum number of blocks; two with the channels-last loaders at 128 x 128, whose 100 bytes of spills cost less than the second block gives:
+// 32 x 130 x 56 x 56 -> 129 3x3 input gradient 1990 us without, 1650 with. A minimum of one lets the compiler spend registers freely: 155 against 126 for the 128 x 128 weight gradient,
 // so one block per SM and not two, and 5 to 10 % more time in every layout: 32 x 130 x 56 x 56 -> 129 3x3 1945 us -> 2087.)
 template <class L, int BM, int BN, int TM, int TN, int KG = 1>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN) * KG, L::SEQ && BM * BN == 128 * 128 ? 2 : 0) conv_gemm_simt(ConvArgs g) {
@@ -521,13 +522,20 @@ static ConvArgs base_args(const OmtConvGeo* g) {
   return a;
 }
 
+// Whether the loaders that walk the reduction in steps of eight channels pay, for a reduction over c channels: the last step is partly padding, and so
+// are the products of all its taps. One tap costs little against whole sectors; with 3x3 the padding may be 3/5 of the channels (32 x 56 x 56
+// forward, 9 -> 64 channels: 57 -> 74 us, 10 -> 90: 165 -> 125), with more taps a third (5x5 17 -> 33: 225 -> 252, 25 -> 50: even).
+static bool steps_of_eight_pay(int c, int ks) {
+  const int padded = (c + 7) / 8 * 8;
+  return c >= 8 && (ks == 1 || (ks <= 3 ? 5 * padded <= 8 * c : 3 * padded <= 4 * c));
+}
+
 int simt_conv_fwd(const OmtConvGeo* g, const OmtAct* x, const float* w, const float* bias, const OmtAct* y,
                   uint32_t flags, cudaStream_t s) {
   ConvArgs a = base_args(g);
   a.a = view(x); a.b = view(y); a.w = w; a.bias = bias; a.flags = flags;
   a.M = g->n * g->oh * g->ow; a.N = g->co; a.K = g->ci * g->ks * g->ks;
-  // (channels-last on both sides; below 8 input channels a step of 8 would mostly be padding)
-  if (x->sc == 1 && y->sc == 1 && g->ci >= 8) return launch_gemm<FwdCl>(a, a.M, a.N, 1, s, "conv_fwd_simt");
+  if (x->sc == 1 && y->sc == 1 && steps_of_eight_pay(g->ci, g->ks)) return launch_gemm<FwdCl>(a, a.M, a.N, 1, s, "conv_fwd_simt");
   return launch_gemm<Fwd>(a, a.M, a.N, 1, s, "conv_fwd_simt");
 }
 
@@ -631,7 +639,7 @@ int simt_conv_dgrad(const OmtConvGeo* g, const OmtAct* gy, const float* w, const
   int st_ = g->stride;
   int64_t hi = cdiv(g->ih, st_), wi = cdiv(g->iw, st_);  // phase (0,0) is the largest
   a.N = g->ci;
-  if (gy->sc == 1 && dx->sc == 1 && g->co >= 8) return launch_gemm<DgradCl>(a, (int64_t)g->n * hi * wi, a.N, st_ * st_, s, "conv_dgrad_simt");
+  if (gy->sc == 1 && dx->sc == 1 && steps_of_eight_pay(g->co, g->ks)) return launch_gemm<DgradCl>(a, (int64_t)g->n * hi * wi, a.N, st_ * st_, s, "conv_dgrad_simt");
   return launch_gemm<Dgrad>(a, (int64_t)g->n * hi * wi, a.N, st_ * st_, s, "conv_dgrad_simt");
 }
 
@@ -656,8 +664,9 @@ int simt_conv_wgrad(const OmtConvGeo* g, const OmtAct* x, const OmtAct* gy, floa
   a.M = g->co; a.N = g->ci * g->ks * g->ks; a.K = g->n * g->oh * g->ow;
   wgrad_slices(g, &a.slices, &a.kslice);
   a.out = a.slices == 1 ? dw : part;
-  int r = x->sc == 1 && gy->sc == 1 && g->ci >= 8 ? launch_gemm<WgradCl>(a, a.M, a.N, a.slices, s, "conv_wgrad_simt")
-                                                  : launch_gemm<Wgrad>(a, a.M, a.N, a.slices, s, "conv_wgrad_simt");
+  // (columns as (tap, channel): 3 to 7 % slower with few channels, even at 66 and 90, 5 % faster from 130 on)
+  int r = x->sc == 1 && gy->sc == 1 && g->ci >= 96 ? launch_gemm<WgradCl>(a, a.M, a.N, a.slices, s, "conv_wgrad_simt")
+                                                   : launch_gemm<Wgrad>(a, a.M, a.N, a.slices, s, "conv_wgrad_simt");
   if (r != OMT_OK || a.slices == 1) return r;
   int64_t total = (int64_t)a.M * a.N;
   launch(slab_sum_kernel, (unsigned)cdiv(total, 256), 256, 0, s, part, dw, total, a.slices, scale);
