@@ -16,7 +16,7 @@
 namespace omt {
 
 constexpr int CHUNK = 4096;  // SGD: elements per block, 256 threads x 4 float4
-constexpr int ADAM_THREADS = 512, ADAM_TRIPS = 4, ADAM_CHUNK = ADAM_THREADS * ADAM_TRIPS * 4;
+constexpr int ADAM_THREADS = 256, ADAM_TRIPS = 4, ADAM_CHUNK = ADAM_THREADS * ADAM_TRIPS * 4;
 
 struct DevParam {
   float* p;
@@ -114,9 +114,9 @@ __device__ __forceinline__ void adam_one(const AdamH& h, float bc1, float sbc2, 
 
 // HBM-bound: four streams read and three written, 28 bytes per parameter. A thread has the next trip's four vectors in flight while
 // it computes one, from before the bias corrections are known (one thread per block takes the two powers); the streams do not
-// stay in cache behind it. 64 M parameters in 160 tensors: 329 -> 273 us, 6.57 TB/s (256 threads, no vectors ahead: 317;
-// without the streaming hints 313).
-__global__ void __launch_bounds__(ADAM_THREADS, 2) adam_kernel(const DevParam* __restrict__ table, int count, AdamH h) {
+// stay in cache behind it. 64 M parameters in 160 tensors: 277 -> 270 us, 6.6 TB/s; 100 tensors of 4097: 8.6 -> 6.5. Blocks of 256: with 512
+// the large list is as fast, but many small tensors leave most of a block idle (2000 of 100: 24 us against 19; 500 of 1000: 8.2 against 5.9).
+__global__ void __launch_bounds__(ADAM_THREADS, 4) adam_kernel(const DevParam* __restrict__ table, int count, AdamH h) {
   pdl_wait();
   __shared__ float corr[2];
   const DevParam t = table[find_tensor_warp(table, count, blockIdx.x)];

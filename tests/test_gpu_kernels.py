@@ -1162,3 +1162,29 @@ def test_weight_relayout_on_both_sides_of_its_lines(capi, case):
 def test_exact_float32_convolutions_around_the_lines_of_their_loaders(capi, case):
     """Channel counts on both sides of where the channels-last loaders take over, bounded as in test_exact_float32_convolutions_vs_aten."""
     test_exact_float32_convolutions_vs_aten(capi, case, True)
+
+
+@pytest.mark.parametrize("shift", [0, 1], ids=["aligned", "shifted"])
+@pytest.mark.parametrize("decoupled", [False, True], ids=["adam", "adamw"])
+def test_adam_over_ragged_tables(capi, decoupled, shift):
+    """Sizes around a vector, a trip and a block's share of the elements, on a 16-byte boundary and 4 bytes past it, in tables around the 32 and 1024
+    entries that a step of the search covers, vs the oracle."""
+    rng = np.random.default_rng(3)
+    ragged = [1, 3, 4, 0, 1023, 1024, 1025, 2047, 2048, 2049, 4095, 4096, 4097, 8191, 8192, 8193, 16385, 2, 5, 12289]
+    for sizes in (ragged, [7] * 31, [4096, 5] * 16, [4097] + [5] * 32, [5, 1, 9, 4100, 3] * 205):
+        offs, n = [], 0
+        for k in sizes:
+            offs.append(n + shift)
+            n += (k + 7) // 4 * 4
+        h = [rng.standard_normal(n).astype(np.float32) for _ in range(3)] + [rng.random(n).astype(np.float32)]
+        d = [torch.from_numpy(a).cuda() for a in h]
+        view = lambda a: [a[o:o + k] for o, k in zip(offs, sizes)]
+        steps = [torch.full((), 1.0 + i % 5, device="cuda") for i in range(len(sizes))]
+        p, g, m, v = (view(a) for a in d)
+        capi.adam(p, g, m, v, steps, 1e-2, weight_decay=0.1, decoupled=decoupled)
+        want = [a.copy() for a in h]
+        for i, (pp, gg, mm, vv) in enumerate(zip(*(view(a) for a in want))):
+            if pp.size:
+                oracle.c.adam(pp, gg, mm, vv, 1.0 + i % 5, 1e-2, wd=0.1, decoupled=decoupled)
+        for got, ref in zip(d, want):  # (also the gaps between the tensors, which nothing may touch)
+            assert rel_err(host(got), ref) <= 1e-6
