@@ -202,6 +202,8 @@ int omt_conv_bias_grad(const OmtAct* gy, int32_t n, int32_t c, int32_t h, int32_
  * average pooling, its broadcast's gradient, and the bias gradient of a Linear layer (one image of `rows` pixels). The
  * reference reduces these with its generic kernels (csrc/reduce.cpp:1-127). */
 int omt_channel_sum(const float* x, int32_t images, int64_t pixels, int32_t c, int32_t mean, float* out, omt_stream_t stream);
+/* 1 where omt_channel_sum is the faster way to take these sums, 0 where a general reduction is (and for what it does not take). */
+int omt_channel_sum_pays(const float* x, int32_t images, int64_t pixels, int32_t c);
 
 /* out[M,N] (row-major) = A[M,K] * B[K,N] (+ bias[N]) in float32 on the same tensor-core kernels: a matrix product is the
  * 1x1 case of the implicit GEMM (rows = pixels). Replaces mm_into / mm_ / addmm_ (csrc/linalg.cpp:25-92; the generated

@@ -83,6 +83,7 @@ SIGNATURES = {
     "omt_conv_wgrad_noalloc": (_I, [_G, _A, _A, _P, _F, _P]),
     "omt_conv_bias_grad": (_I, [_A, _I, _I, _I, _I, _P, _F, _P]),
     "omt_channel_sum": (_I, [_P, _I, _I64, _I, _I, _P, _P]),
+    "omt_channel_sum_pays": (_I, [_P, _I, _I64, _I]),
     "omt_kernel_timing": (_I, [_I]),
     "omt_kernel_times": (_SZ, [C.c_char_p, _SZ, _I]),
     "omt_gemm": (_I, [_P, _I64, _I64, _P, _I64, _I64, _P, _P, _I, _I, _I, _P]),
@@ -128,7 +129,7 @@ SIGNATURES = {
     "omt_act_copy": (_I, [_A, _A, _I, _I, _I, _I, _P]),
 }
 # these return a status that is not an error code convention (counts, booleans)
-_UNCHECKED = {"omt_device", "omt_last_error", "omt_stream_query", "omt_event_query"}
+_UNCHECKED = {"omt_channel_sum_pays", "omt_device", "omt_last_error", "omt_stream_query", "omt_event_query"}
 
 _lib = None
 

@@ -149,7 +149,7 @@ static Tensor adaptive_avg_pool2d_(const Tensor& x_, IntArrayRef os) {
   NEED(f32(x_) && x_.dim() == 4 && x_.numel() > 0 && os[0] > 0 && os[1] > 0, "adaptive avg pool: 4-D float32");
   Tensor x = dense4(x_);
   Tensor out = dense4(empty_dev({x.size(0), x.size(1), os[0], os[1]}, at::kFloat, is_cl(x) && os[0] * os[1] > 1));
-  if (os[0] * os[1] == 1 && layout4(x) == 1 && x.size(0) <= 65535) {
+  if (os[0] * os[1] == 1 && layout4(x) == 1 && channel_sum_pays(x, x.size(0), x.size(2) * x.size(3), x.size(1))) {
     check(omt_channel_sum(fptr(x), (int)x.size(0), x.size(2) * x.size(3), (int)x.size(1), 1, out.data_ptr<float>(), cur_stream()), "global avg pool");
     return out;
   }
@@ -170,20 +170,20 @@ static Tensor adaptive_avg_pool2d_backward_(const Tensor& gy_, const Tensor& x) 
 }
 
 // Sums and means over the pixels of channels-last images (global pooling in eager code is a mean, the gradient of a per-channel
-// gate a sum) and over the rows of a matrix (the bias gradient of nn.Linear) are channel sums; every other reduction goes to
-// ATen's CUDA kernel over the bridge, as all of them did. A MobileNetV3 step has 21 of them
+// gate a sum) and over the rows of a matrix (the bias gradient of nn.Linear) are channel sums, of the sizes that omt_channel_sum_pays names;
+// every other reduction goes to ATen's CUDA kernel over the bridge, as all of them did. A MobileNetV3 step has 21 of them
 // of about 12 us in ATen's kernel, for a few hundred KB each: 3632 -> 3575 us.
 static bool channel_sum(const Tensor& x, at::OptionalIntArrayRef dim, bool keepdim, std::optional<at::ScalarType> dtype, bool mean, Tensor& out) {
   if (!f32(x) || (dtype && *dtype != at::kFloat) || !dim || x.numel() == 0 || x.numel() >= (1ll << 40)) return false;
   const int64_t R = x.dim();
   auto wrapped = [&](size_t k) { return (*dim)[k] < 0 ? (*dim)[k] + R : (*dim)[k]; };
-  if (R == 2 && dim->size() == 1 && wrapped(0) == 0 && x.is_contiguous() && x.size(0) > 1 && x.size(1) < (1ll << 31)) {
+  if (R == 2 && dim->size() == 1 && wrapped(0) == 0 && x.is_contiguous() && x.size(0) > 1 && channel_sum_pays(x, 1, x.size(0), x.size(1))) {
     out = keepdim ? empty_dev({1, x.size(1)}, at::kFloat) : empty_dev({x.size(1)}, at::kFloat);
     check(omt_channel_sum(fptr(x), 1, x.size(0), (int)x.size(1), mean, out.data_ptr<float>(), cur_stream()), "sum over rows");
     return true;
   }
-  if (R == 4 && dim->size() == 2 && wrapped(0) + wrapped(1) == 5 && (wrapped(0) == 2 || wrapped(0) == 3) && layout4(x) == 1 && x.size(0) <= 65535 &&
-      x.size(1) < (1ll << 31)) {
+  if (R == 4 && dim->size() == 2 && wrapped(0) + wrapped(1) == 5 && (wrapped(0) == 2 || wrapped(0) == 3) && layout4(x) == 1 &&
+      channel_sum_pays(x, x.size(0), x.size(2) * x.size(3), x.size(1))) {
     out = keepdim ? empty_dev({x.size(0), x.size(1), 1, 1}, at::kFloat) : empty_dev({x.size(0), x.size(1)}, at::kFloat);
     check(omt_channel_sum(fptr(x), (int)x.size(0), x.size(2) * x.size(3), (int)x.size(1), mean, out.data_ptr<float>(), cur_stream()), "sum over pixels");
     return true;

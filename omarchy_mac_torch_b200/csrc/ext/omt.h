@@ -76,6 +76,9 @@ Tensor to_layout(const Tensor& t, int layout);
 inline OmtAct act(const Tensor& t) {
   return OmtAct{t.data_ptr<float>(), t.stride(0), t.stride(1), t.stride(2), t.stride(3)};
 }
+inline bool channel_sum_pays(const Tensor& x, int64_t images, int64_t pixels, int64_t c) {
+  return images <= 65535 && c < (1ll << 31) && omt_channel_sum_pays(x.data_ptr<float>(), (int)images, pixels, (int)c) == 1;
+}
 inline OmtAct null_act() { return OmtAct{nullptr, 0, 0, 0, 0}; }
 Tensor contig(const Tensor& t);  // contiguous (any dtype), on the device
 

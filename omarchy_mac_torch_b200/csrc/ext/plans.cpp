@@ -215,7 +215,7 @@ static Tensor plan_forward(Plan& p, const Tensor& x_) {
       cur = y;
     } else {  // gap
       Tensor y = empty_dev({n, c, 1, 1}, at::kFloat);
-      if (layout4(cur) == 1 && n <= 65535) {
+      if (layout4(cur) == 1 && channel_sum_pays(cur, n, (int64_t)h * w, c)) {
         check(omt_channel_sum(fptr(cur), n, (int64_t)h * w, c, 1, y.data_ptr<float>(), cur_stream()), "plan global avg pool");
       } else {
         OmtAct ax = act(cur), ay = act(y);

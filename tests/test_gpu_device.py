@@ -887,3 +887,22 @@ def test_fused_pointwise_long_programs_on_both_sides_of_the_vector_line(omt):
             whole = [t[1:].clone() for t in src]
             assert torch.equal(fp(f"pw1|2|{chain}|{0.5.hex()}", whole).cpu(), fp(f"pw1|2|{chain}|{0.5.hex()}", [t[1:] for t in src]).cpu()), (k, n)
     assert not omt.FALLBACKS, dict(omt.FALLBACKS)
+
+
+@pytest.mark.parametrize("shape,ours", [((32, 72, 8, 8), True), ((16, 2048, 7, 7), True), ((600, 16, 3, 3), False), ((3000, 4, 2, 2), False), ((37, 2048, 7, 7), True), ((38, 2048, 7, 7), False), ((1, 33, 90, 90), False),
+                                        ((20, 7, 16, 16), True), ((64, 100), True), ((128, 1001), True), ((513, 257), False), ((16, 200_000), False), ((4096, 64), True), ((60_000, 33), False)], ids=lambda s: "x".join(map(str, s)) if isinstance(s, tuple) else None)
+def test_channel_sums_only_where_they_are_faster(omt, shape, ours):
+    """Which sums over pixels and rows run on the channel-sum kernel, and the values of both ways against float64 (the bound of a float32 sum of k
+    terms, k 2^-24 of the sum of absolute values)."""
+    from omarchy_mac_torch_b200.native import core
+    x = torch.randn(shape)
+    if len(shape) == 4:
+        x = x.contiguous(memory_format=torch.channels_last)
+    dims = (2, 3) if len(shape) == 4 else (0,)
+    d = x.to(D)
+    k = shape[2] * shape[3] if len(shape) == 4 else shape[0]
+    for fn in [lambda t: t.sum(dims), lambda t: t.mean(dims)] + ([lambda t: F.adaptive_avg_pool2d(t, 1)] if len(shape) == 4 else []):
+        core.kernel_counts(True)
+        got = fn(d)
+        assert (core.kernel_counts(False).get("channel_sum_nhwc", 0) > 0) == ours
+        assert ((got.cpu().double() - fn(x.double())).abs() <= (k + 2) * 2.0**-24 * fn(x.double().abs())).all()
