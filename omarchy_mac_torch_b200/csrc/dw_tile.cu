@@ -10,8 +10,8 @@
 // channel pairs of one pixel: 128 contiguous bytes, no bank conflicts, whole sectors in global memory.
 // The copies are 16 bytes when c % 4 == 0 and the tensors are 16-byte aligned (weight gradient only: see the dispatch in dw.cu), else
 // 4 bytes (32 lanes = one pixel's slab).
-// What bounds them: issue, at two blocks per SM. Forward 5x5 on 64 x 96 x 56 x 56 with 16-byte copies issued in 53 % of the cycles
-// with 3.3 warps per scheduler, the largest stall being a sum's own previous multiply-add; DRAM was at 17 %.
+// What bounds them: issue, at two blocks per SM. Forward 5x5 on 128 x 97 x 56 x 56 (274 us) issues in 57 % of the cycles with 3.4 warps per
+// scheduler; the largest stall is a sum's own previous multiply-add, then the row barrier; DRAM is at 12 %.
 #include <algorithm>
 #include <mutex>
 
@@ -403,7 +403,12 @@ int dw_tile_wgrad(const DwArgs& a, bool vec, float scale, float* dw, omt_stream_
   const int64_t resident = std::max<int64_t>(1, (int64_t)per_sm * sm_count() / slabs);  // blocks per slab that run at once
   const TilePlan p = plan_tiles(a, 4 * resident * slabs, a.ks + 1);
   const int64_t small = std::max<int64_t>(1, std::min<int64_t>(4, TILE_THREADS / (16 * p.G * p.Z)));  // blocks of few threads: more per SM (27 x 301 x 23 x 21 7x7 stride 2 110 -> 63 us, 64 x 96 x 56 x 56 77 -> 52)
-  const int SL = (int)std::min<int64_t>(resident * small, (int64_t)p.imgs * p.segs * p.xtiles);
+  // Every thread adds its share of the output pixels one after the other in float32. 7x7 takes up to four times the blocks, one after the other on an SM,
+  // to keep that share to about 192: 128 x 96 x 56 x 56 4.3e-7 of the float64 result without, 2.5e-7 with, 3.5e-7 in the kernel that this one replaces, at
+  // 198 -> 208 us. (3x3 and 5x5 have shorter shares, two blocks being resident, and are within a tenth of the error of the kernels they replace, or below it.)
+  const int64_t items = (int64_t)p.imgs * p.segs * p.xtiles, once = std::min(resident * small, items);
+  const int64_t rounds = a.ks == 7 ? std::min<int64_t>(4, std::max<int64_t>(1, std::min(cdiv((int64_t)a.n * a.oh * a.ow, once * p.G * p.Z * 192), items / once))) : 1;
+  const int SL = (int)(once * rounds);
   const int kk = a.ks * a.ks;
   Scratch sc;
   int r = sc.get(nullptr, 0, (size_t)a.c * SL * kk * sizeof(float), stream);

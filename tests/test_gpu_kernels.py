@@ -1188,3 +1188,16 @@ def test_adam_over_ragged_tables(capi, decoupled, shift):
                 oracle.c.adam(pp, gg, mm, vv, 1.0 + i % 5, 1e-2, wd=0.1, decoupled=decoupled)
         for got, ref in zip(d, want):  # (also the gaps between the tensors, which nothing may touch)
             assert rel_err(host(got), ref) <= 1e-6
+
+
+@pytest.mark.parametrize("n,c,h", [(128, 96, 56), (2, 130, 224), (64, 66, 57)])
+def test_depthwise_7x7_weight_gradient_adds_in_short_chains(capi, n, c, h):
+    """At most about 192 products one after the other: rounding each of m partial sums of random terms leaves u sqrt(m / 2) of the result, where u, the
+    root mean square of a rounding relative to the sum, is below 2^-25."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x, gy = (torch.randn(n, h, h, c, device="cuda", generator=gen).permute(0, 3, 1, 2) for _ in range(2))
+    got = capi.dw_wgrad(x, gy, 7, 1, 3).double()
+    want = torch.zeros_like(got)
+    for i in range(0, n, 8):
+        want += depthwise_inside(x[i:i + 8].double(), torch.zeros_like(want), gy[i:i + 8].double(), 1, 3)[2]
+    assert (got - want).norm() <= 2.0**-25 * (192 / 2) ** 0.5 * want.norm()
