@@ -342,9 +342,11 @@ __global__ void __launch_bounds__(256) maxpool_bwd_nhwc4_fixed_kernel(PoolArgs a
 // Stride 2: one thread takes an even-aligned 2 x 2 block of input pixels. The block meets at most two windows per axis, whose
 // indices and gradients are loaded once and serve all four pixels: 4 window loads per block instead of 9 per-pixel ones
 // (this kernel is bound by the bytes that cross L1, not by HBM). Indices are compared in 32 bits (h * w < 2^31).
-// Five blocks per SM are asked for with 3x3: left alone the compiler takes 56 registers, which is four (256 x 64 x 112 x 112: 338 us, 301 with five).
+// Blocks of 128: the kernel takes 56 registers, so nine of them fit an SM where four of 256 do (256 x 64 x 112 x 112, 3x3: 338 us with 256 threads,
+// 316 with 256 held to 48 registers, 295 so).
+constexpr int S2_THREADS = 128;
 template <int KS>
-__global__ void __launch_bounds__(256, KS == 3 ? 5 : 0) maxpool_bwd_nhwc4_s2_block_kernel(PoolArgs a, const int64_t* __restrict__ idx) {
+__global__ void __launch_bounds__(S2_THREADS, 9) maxpool_bwd_nhwc4_s2_block_kernel(PoolArgs a, const int64_t* __restrict__ idx) {
   pdl_wait();
   const int c4 = a.c >> 2, hb = (a.ih + 1) >> 1, wb = (a.iw + 1) >> 1;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -592,11 +594,11 @@ int omt_maxpool_bwd(const OmtAct* gy, const int64_t* idx, const OmtAct* gx, int3
     const bool square = p->kh == p->kw && p->sh == p->sw && p->dh == 1 && p->dw == 1;
     const int64_t blocks2 = (int64_t)n * ((ih + 1) / 2) * ((iw + 1) / 2) * (c / 4);  // 2 x 2 pixel blocks x channel quads
     if (square && p->kh == 3 && p->sh == 2 && iw > 1) {
-      launch(maxpool_bwd_nhwc4_s2_block_kernel<3>, (unsigned)cdiv(blocks2, 256), 256, 0, st(stream), pa(gy, gx, n, c, ih, iw, oh, ow, p, 0, 0), idx);
+      launch(maxpool_bwd_nhwc4_s2_block_kernel<3>, (unsigned)cdiv(blocks2, S2_THREADS), S2_THREADS, 0, st(stream), pa(gy, gx, n, c, ih, iw, oh, ow, p, 0, 0), idx);
       return check_launch("maxpool_bwd_nhwc4_k3s2");
     }
     if (square && p->kh == 2 && p->sh == 2 && iw > 1) {
-      launch(maxpool_bwd_nhwc4_s2_block_kernel<2>, (unsigned)cdiv(blocks2, 256), 256, 0, st(stream), pa(gy, gx, n, c, ih, iw, oh, ow, p, 0, 0), idx);
+      launch(maxpool_bwd_nhwc4_s2_block_kernel<2>, (unsigned)cdiv(blocks2, S2_THREADS), S2_THREADS, 0, st(stream), pa(gy, gx, n, c, ih, iw, oh, ow, p, 0, 0), idx);
       return check_launch("maxpool_bwd_nhwc4_k2s2");
     }
     launch(maxpool_bwd_nhwc4_kernel, (unsigned)cdiv(total, 256), 256, 0, st(stream), pa(gy, gx, n, c, ih, iw, oh, ow, p, 0, 0), idx);
