@@ -925,12 +925,12 @@ __global__ void __launch_bounds__(256) weight_split_kernel(const float* __restri
 // taps, or in dgrad rows x taps, of the original) and the writes (32 channels of one tap) are contiguous. A block reads all taps of its rows, so
 // it is no kernel for a stride phase.
 constexpr int SPLIT_FLOATS = 4096;
-constexpr int split_rows(int kk) { return kk == 1 ? 8 : (kk <= 9 ? 4 : (kk <= 49 ? 2 : 1)); }  // many small blocks; 32 * (split_rows(kk) * kk | 1) <= SPLIT_FLOATS up to 11 x 11
+constexpr int split_rows(int kk) { return kk <= 9 ? 4 : (kk <= 49 ? 2 : 1); }  // many small blocks; 32 * (split_rows(kk) * kk | 1) <= SPLIT_FLOATS up to 11 x 11
 template <bool DGRAD>
 __global__ void __launch_bounds__(256) weight_split_tile_kernel(const float* __restrict__ w, float* __restrict__ out, SplitArgs a, int RB, const BnFold f) {
   pdl_wait();
   __shared__ float sm[SPLIT_FLOATS];
-  __shared__ float scale[8];  // of the tile's rows
+  __shared__ float scale[4];  // of the tile's rows
   const int kk = a.ks * a.ks, rows = DGRAD ? a.ci : a.co, chans = DGRAD ? a.co : a.ci;
   const uint32_t cblocks = a.cpad / 32;  // one grid dimension for both: either extent may be far beyond 65535 (the columns of a matrix product)
   const int r0 = (int)(blockIdx.x / cblocks) * RB, c0 = (int)(blockIdx.x % cblocks) * 32, tid = threadIdx.x;
@@ -991,10 +991,11 @@ __global__ void __launch_bounds__(256) weight_split_1x1_kernel(const float* __re
   *reinterpret_cast<float4*>(o) = make_float4(hi[0], hi[1], hi[2], hi[3]);
   *reinterpret_cast<float4*>(o + (int64_t)a.co * a.cpad) = make_float4(lo[0], lo[1], lo[2], lo[3]);
 }
-// Tiles where their contiguous reads outweigh two passes through a block (element by element -> tiles, warm): a whole filter of 3x3 and more
-// with 2^16 rows x channels and more (512 x 512 3x3 16.2 -> 13.4 us, 256 x 256 5.2 -> 5.0, but 64 x 64 1.7 -> 2.9), and the transposition of
-// a 1x1 filter below 2^18 (256 x 256 2.2 -> 1.8, but 2048 x 2048 28.6 -> 32.6). A stride phase of a 512 x 512 3x3 filter: 3.3 -> 7.2 us with one tap, 8.4 ->
-// 9.8 with four. These ratios hold with L2 flushed.
+// Tiles where their contiguous reads and their one scale per row outweigh two passes through a block (element by element -> tiles, warm; with L2 flushed the
+// ratios are the same or nearer to one): whole filters of several taps with 2^17 rows x channels and more, input gradients (512 x 512 3x3 14.8 -> 14.3 us,
+// 1000 x 512 5x5 80 -> 70; 256 x 256 3x3 4.9 -> 5.4, 64 x 64 1.7 -> 3.0), folded forward layers (14.9 -> 14.3, 76 -> 68; 4.9 -> 5.3, 1.8 -> 3.4) and forward layers
+// beyond 3x3 (70 -> 66; 3x3 13.3 -> 13.8, 2048 x 512 51.5 -> 50.4). Not 1x1 (256 x 256 input gradient 2.1 -> 1.9, but 512 x 512 3.1 -> 3.5 and 2048 x 2048 25 ->
+// 36), nor the stride phases of a filter, of which a block would read all taps (512 x 512 3x3, 2x2 taps of it: 7.5 -> 10.1).
 static int split_weights(const float* w, float* out, const SplitArgs& a, const BnFold* fold, cudaStream_t s) {
   const int rows = a.dgrad ? a.ci : a.co, chans = a.dgrad ? a.co : a.ci, RB = split_rows(a.ks * a.ks);
   const BnFold f = fold ? *fold : BnFold{};
@@ -1003,7 +1004,7 @@ static int split_weights(const float* w, float* out, const SplitArgs& a, const B
     return check_launch("conv_tc_weight_split");
   }
   const int64_t elements = (int64_t)rows * chans;
-  if (!a.window && a.kh == a.ks && a.kw == a.ks && (a.ks == 1 ? a.dgrad && elements < 1 << 18 : elements >= 1 << 16)) {
+  if (!a.window && a.ks > 1 && a.kh == a.ks && a.kw == a.ks && elements >= 1 << 17 && (a.dgrad || f.gamma || a.ks > 3)) {
     const unsigned grid = (unsigned)((int64_t)(a.cpad / 32) * cdiv(rows, RB));
     if (a.dgrad) launch(weight_split_tile_kernel<true>, grid, 256, 0, s, w, out, a, RB, f);
     else launch(weight_split_tile_kernel<false>, grid, 256, 0, s, w, out, a, RB, f);

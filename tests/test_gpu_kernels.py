@@ -1127,11 +1127,11 @@ def test_depthwise_kernels_on_both_sides_of_their_lines(capi, case):
         assert ((v.double() - ref).abs() <= (k + 2) * 2.0**-24 * bound + 1e-30).all()
 
 
-@pytest.mark.parametrize("case", [(2, 16, 4096, 3, 3, 3, 1, 1), (1, 16, 4095, 3, 3, 3, 1, 1), (1, 264, 260, 4, 5, 3, 1, 1), (1, 40, 1700, 3, 4, 5, 1, 2), (1, 272, 264, 5, 5, 3, 2, 1), (2, 264, 252, 3, 3, 11, 1, 5),
-                                  (3, 512, 512, 2, 2, 1, 1, 0), (3, 512, 508, 2, 2, 1, 1, 0), (1, 260, 256, 4, 4, 2, 1, 0)], ids=lambda t: "x".join(map(str, t)))
+@pytest.mark.parametrize("case", [(2, 32, 4096, 3, 3, 3, 1, 1), (1, 32, 4095, 3, 3, 3, 1, 1), (1, 264, 260, 4, 5, 3, 1, 1), (1, 40, 3300, 3, 4, 5, 1, 2), (1, 272, 484, 5, 5, 3, 2, 1), (2, 264, 500, 3, 3, 11, 1, 5),
+                                  (3, 512, 512, 2, 2, 1, 1, 0), (3, 260, 36, 2, 2, 1, 1, 0), (1, 520, 256, 4, 4, 2, 1, 0)], ids=lambda t: "x".join(map(str, t)))
 def test_weight_relayout_on_both_sides_of_its_lines(capi, case):
-    """Rows x channels at 2^16 (filters of several taps) and 2^18 (1x1 input gradients), stride phases, ragged edges: forward, the same with a folded
-    BatchNorm, and input gradient against float64 (TOL, the path's own bound), and that tiles run where the sizes say so."""
+    """Rows x channels at 2^17, filters of one and several taps, stride phases, ragged edges: forward, the same with a folded BatchNorm, and input
+    gradient against float64 (TOL, the path's own bound), and that tiles run where the sizes say so."""
     n, ci, co, h, w, ks, s, p = case
     gen = torch.Generator().manual_seed(sum(case))
     x, wt, b = torch.randn(n, ci, h, w, generator=gen), torch.randn(co, ci, ks, ks, generator=gen) / (ci * ks * ks) ** 0.5, torch.randn(co, generator=gen)
@@ -1142,19 +1142,19 @@ def test_weight_relayout_on_both_sides_of_its_lines(capi, case):
     gy = torch.randn(y.shape, generator=gen)
     dx, = torch.autograd.grad(y, [xd], gy.double())
     y = y.detach()
-    tiles = (ks > 1 and ci * co >= 2**16, (ks > 1 and s == 1 and ci * co >= 2**16) or (ks == 1 and ci * co < 2**18))
-    capi.kernel_counts(reset=True)
+    big = ks > 1 and ci * co >= 2**17
+    tiles = lambda: capi.kernel_counts(reset=True).get("conv_tc_weight_split_tiles", 0) > 0
+    tiles()
     got = capi.conv_fwd(dev(x, True), wt.cuda(), b.cuda(), s, p, flags=capi.FORCE_TC, cl=True)
-    assert rel_err(host(got), y.numpy()) <= TOL and (capi.kernel_counts(reset=True).get("conv_tc_weight_split_tiles", 0) > 0) == tiles[0]
+    assert rel_err(host(got), y.numpy()) <= TOL and tiles() == (big and ks > 3)
     got = torch.full_like(got, float("nan"))
     q = [v.cuda() for v in (wt, b, gamma, beta, rm, rv)]
     capi.call("omt_conv_fwd_bn", capi.geo(n, ci, co, h, w, ks, s, p), capi.act(dev(x, True)), *map(capi.ptr, q), 1e-5, capi.act(got), 0, capi.stream_handle())
     k = (gamma.double() / (rv.double() + 1e-5).sqrt()).view(1, -1, 1, 1)
-    assert rel_err(host(got), ((y - rm.double().view(1, -1, 1, 1)) * k + beta.double().view(1, -1, 1, 1)).numpy()) <= TOL
+    assert rel_err(host(got), ((y - rm.double().view(1, -1, 1, 1)) * k + beta.double().view(1, -1, 1, 1)).numpy()) <= TOL and tiles() == big
     if co % 4 == 0:
-        capi.kernel_counts(reset=True)
         assert rel_err(host(capi.conv_dgrad(dev(gy, True), wt.cuda(), (h, w), s, p, flags=capi.FORCE_TC, cl=True)), dx.numpy()) <= TOL
-        assert (capi.kernel_counts().get("conv_tc_weight_split_tiles", 0) > 0) == tiles[1]
+        assert tiles() == (big and s == 1)
 
 
 @pytest.mark.parametrize("case", [(2, 9, 12, 20, 19, 3, 1, 1), (2, 10, 14, 20, 19, 3, 1, 1), (2, 17, 18, 15, 16, 5, 1, 2), (2, 18, 17, 15, 16, 5, 2, 2), (3, 9, 9, 30, 31, 1, 1, 0), (2, 95, 20, 11, 12, 3, 1, 1), (2, 97, 20, 11, 12, 3, 2, 1)],
