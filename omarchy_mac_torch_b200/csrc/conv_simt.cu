@@ -664,8 +664,8 @@ int simt_conv_wgrad(const OmtConvGeo* g, const OmtAct* x, const OmtAct* gy, floa
   a.M = g->co; a.N = g->ci * g->ks * g->ks; a.K = g->n * g->oh * g->ow;
   wgrad_slices(g, &a.slices, &a.kslice);
   a.out = a.slices == 1 ? dw : part;
-  // (columns as (tap, channel): 3 to 7 % slower with few channels, even at 66 and 90, 5 % faster from 130 on)
-  int r = x->sc == 1 && gy->sc == 1 && g->ci >= 96 ? launch_gemm<WgradCl>(a, a.M, a.N, a.slices, s, "conv_wgrad_simt")
+  // (columns as (tap, channel): 3 to 7 % slower below, even around 66, 1 to 3 % faster at 90 where there are pixels enough, 5 % from 130 on)
+  int r = x->sc == 1 && gy->sc == 1 && g->ci >= 64 ? launch_gemm<WgradCl>(a, a.M, a.N, a.slices, s, "conv_wgrad_simt")
                                                    : launch_gemm<Wgrad>(a, a.M, a.N, a.slices, s, "conv_wgrad_simt");
   if (r != OMT_OK || a.slices == 1) return r;
   int64_t total = (int64_t)a.M * a.N;
