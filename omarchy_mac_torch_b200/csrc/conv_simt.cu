@@ -335,11 +335,12 @@ struct WgradCl : Wgrad {
 // outputs over very many pixels (16 x 32 outputs, eight groups), which a 128 x 64 tile computes almost entirely as padding: 252 us
 // for 16 x 27 outputs over 401 408 pixels, 7 % of a MobileNetV3 step. With the channels-last loaders the three passes of a
 // 90 -> 50 channel 3x3 stride-2 layer (13 x 57 x 43) go from 217 to 151 us, that step from 3783 to 3592.
-// (0: no minimum number of blocks; two with the channels-last loaders at 128 x 128, whose 100 bytes of spills cost less than the second block gives:
-// 32 x 130 x 56 x 56 -> 129 3x3 input gradient 1990 us without, 1650 with. A minimum of one lets the compiler spend registers freely: 155 against 126 for the 128 x 128 weight gradient,
-// so one block per SM and not two, and 5 to 10 % more time in every layout: 32 x 130 x 56 x 56 -> 129 3x3 1945 us -> 2087.)
+// The minimum number of blocks: none as a rule, for a minimum of one lets the compiler spend registers freely (155 against 126 for the 128 x 128 weight
+// gradient, so one block per SM and not two: 32 x 130 x 56 x 56 -> 129 3x3 1945 us -> 2087). One where two groups share a tile, as those launches have no second
+// block for an SM (8 x 50 x 7 x 7 -> 250 3x3 input gradient 129 us -> 113). Two with the channels-last loaders at 128 x 128, whose 100 bytes of spills cost less
+// than the second block gives (32 x 130 x 56 x 56 -> 129 3x3 input gradient 1990 us -> 1650).
 template <class L, int BM, int BN, int TM, int TN, int KG = 1>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN) * KG, L::SEQ && BM * BN == 128 * 128 ? 2 : 0) conv_gemm_simt(ConvArgs g) {
+__global__ void __launch_bounds__((BM / TM) * (BN / TN) * KG, L::SEQ && BM * BN == 128 * 128 ? 2 : (KG == 2 ? 1 : 0)) conv_gemm_simt(ConvArgs g) {
   pdl_wait();
   constexpr int TY = BM / TM, GM = TM / 4, GN = TN / 4, TG = (BM / TM) * (BN / TN);
   constexpr bool A_MF = L::A_MFAST && TG == 256, B_NF = L::B_NFAST && TG == 256;  // small groups: lanes along k, one position per thread
